@@ -28,9 +28,10 @@ _REFERENCE_SRC_DEFAULT = "/root/reference"
 
 
 def reference_sources() -> str | None:
-    """The directory holding the reference's sources, or None where it is absent."""
+    """The directory holding the reference's sources, or None where it is absent
+    or holds none (an empty mount point)."""
     d = os.environ.get("KCLPP_REFERENCE_SRC", _REFERENCE_SRC_DEFAULT)
-    return d if os.path.isdir(d) else None
+    return d if os.path.isfile(os.path.join(d, "kCDensestNoAtom.c")) else None
 
 
 def build(ref: bool = False, ref_if_present: bool = False) -> None:
