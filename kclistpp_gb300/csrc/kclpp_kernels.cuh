@@ -35,6 +35,7 @@
 #pragma once
 
 #include <mutex>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -485,10 +486,24 @@ __device__ __forceinline__ uint32_t triangles_in(const Bits<1> &P, const uint32_
   return c;
 }
 
+constexpr int kPairMembers = 256;  // most members of PairLevel's I
+// Words of PairLevel's per-warp scratch: P's words, a group's row offsets and (value,
+// range) pairs, I's values, increments and positions, the members of P.
+__host__ __device__ inline size_t pair_words(uint32_t dmax) {
+  return 32 + 32 + 64 + kPairMembers + kPairMembers / 4 + kPairMembers / 2 + (((size_t)dmax + 7) / 8) * 4;
+}
+
+// Words of a Seq warp: the stream's values or increments (dmax + 1), and with
+// rows in shared memory at k >= 4 the last two levels' scratch.  At k = 4 a
+// stream uses one or the other, so they share the words.
+__host__ __device__ inline size_t seq_warp_words(int k, uint32_t dmax, bool rows_in_smem) {
+  const size_t v = ((size_t)dmax + 4) / 4 * 4, p = k >= 4 && rows_in_smem ? pair_words(dmax) : 0;
+  return k == 4 ? (v > p ? v : p) : v + p;
+}
 // Shared-memory layout of a tier M / L CTA (dmax = largest out-degree the
 // launch allows, NW warps).  Tier L keeps `rows` in a global slab instead.
 struct LayoutM {
-  size_t list, rows, base, acc, rank, inv, dl, cbuf, total;
+  size_t list, rows, base, acc, rel, rank, inv, dl, cbuf, total;
 };
 // Per-warp scratch of the k = 4 counting path (edges_in): P's words and its
 // members, compacted.
@@ -505,7 +520,8 @@ __host__ __device__ inline LayoutM layout_m(int mode, int k, uint32_t dmax, int 
   L.acc = at; if (mode == MODE_SEQ) at = align16(at + (size_t)(dmax + 1) * 8);
   L.rank = at; if (mode == MODE_ORDER) at = align16(at + (size_t)dmax * 2);
   L.inv = at; if (mode == MODE_ORDER) at = align16(at + (size_t)dmax * 2);
-  L.dl = at; if (mode == MODE_SEQ) at = align16(at + (size_t)nw * (dmax + 1) * 4);
+  L.rel = at; if (mode == MODE_SEQ && k >= 4 && rows_in_smem) at = align16(at + (size_t)(dmax + 1) * 4);
+  L.dl = at; if (mode == MODE_SEQ) at = align16(at + (size_t)nw * seq_warp_words(k, dmax, rows_in_smem) * 4);
   L.cbuf = at;
   if (mode != MODE_SEQ && (k == 4 || k == 5) && rows_in_smem) at = align16(at + (size_t)nw * cbuf_words(dmax) * 4);
   L.total = at;
@@ -689,16 +705,681 @@ __device__ __forceinline__ typename VA::T value_of(int x, const VA &va, int lane
   return __shfl_sync(KCL_FULL, v, x & 31);
 }
 
+// The last two levels of a stream, at once: for u in P ascending, the chain
+// over V = P ∩ row(u) (kCDensestNoAtom.c:173-188), values in 32 bits.
+//
+// What bounds these levels is instruction issue, and a walk over the words of
+// every V spends it on lanes without a candidate and on candidates whose fate
+// is known.  A member whose value is at or above c + |P| (|P| - 1) / 2 -- c
+// plus every clique of the call -- can never be below a prefix value: it falls
+// every time and never changes.  Only the others, I, are followed, compacted
+// 32 to a slot.  The members u are taken 32 at a time (lane g: u_g, with
+// tot_g = |V|).
+//
+// A group whose comparisons cannot change their outcome while it runs is
+// settled by counting.  Inside the group i's value stays in [v_i, v_i + S_i],
+// S_i = 32 + (i in the group: tot_i), and the prefix value in [c, c + sum
+// tot].  If every i lies wholly below c (class L) or at or above c + sum tot,
+// every chain of a u outside L gives its unit to exactly the members of V in
+// L, the rest falls to the prefix; a u in L is its own prefix (value v_u, up
+// to v_u + S_u) and is compared the same way with its V.  T_i, in i's lane,
+// has bit g set iff i is in u_g's V, so these are popcounts.  When any two of
+// the compared ranges overlap, the group's chains run one after another.
+//
+// Measured on a trimmed RMAT-18 core (233 K edges, k = 4, loads of 4 passes):
+// 94 % of the groups settle; a pass 3.87 -> 1.47 ms against the word-at-a-time
+// chain alone.  From zero, where nothing settles (k = 5, RMAT-15 with planted
+// communities), 15.0 -> 11.9 ms.  At most 40 registers at k = 4 (48 warps per
+// SM): at 80 (24 warps) the same pass took 2.16 ms.
+// Values of a root as 32-bit offsets from its smallest, capped here (the Seq
+// kernel at k >= 4 with rows in shared memory).
+constexpr uint32_t kRelCap = 0x7ffffff0u;
+
+// A whole stream over at most 32 * S candidates, in registers: member i of C
+// is a bit of a mask and a lane (slot i >> 5), which keeps its value, its
+// neighbours below it (crow) and above it (ccol).  Deeper prefixes are masks,
+// so a level costs no set-up, and the last two levels are settled by counting
+// or walked chain by chain as in PairLevel (whose ranges S_i are here exact
+// counts: i's chances as a candidate and its own chain).  Streams of this size
+// are all there is in sparse graphs: 24 Chung-Lu / Erdos-Renyi graphs at
+// k = 3..7 take 12.9 ms for 2 passes with it, 19.6 ms with PairLevel for every
+// stream, 25.2 ms with the word-at-a-time chain.
+template <int S>
+struct TinyStream {
+  using M = typename std::conditional<S == 1, uint32_t, unsigned long long>::type;
+  uint32_t v[S];
+  M crow[S], ccol[S];
+  int lane;
+
+  static __device__ __forceinline__ int pop(M x) {
+    if constexpr (S == 1) return __popc(x);
+    else return __popcll(x);
+  }
+  static __device__ __forceinline__ int first(M x) {
+    if constexpr (S == 1) return __ffs((int)x) - 1;
+    else return __ffsll((long long)x) - 1;
+  }
+  // x[slot of u] from u's lane.
+  template <typename T>
+  __device__ __forceinline__ T of(const T (&x)[S], int u) const {
+    T y = x[0];
+    if constexpr (S == 2) y = u >= 32 ? x[1] : x[0];
+    return __shfl_sync(KCL_FULL, y, u & 31);
+  }
+  static __device__ __forceinline__ M mask_of(const bool (&b)[S]) {
+    M m = __ballot_sync(KCL_FULL, b[0]);
+    if constexpr (S == 2) m |= (M)__ballot_sync(KCL_FULL, b[1]) << 32;
+    return m;
+  }
+  __device__ __forceinline__ bool in(M x, int q) const { return (x >> (32 * q + lane)) & 1u; }
+
+  // list: C's members; the rows are read word by word, a lane per candidate.
+  __device__ __forceinline__ void load(const uint32_t *rows, const uint16_t *list, int nc, const uint32_t *rel) {
+    const uint32_t *col[S];
+    uint32_t bit[S], off[S];
+#pragma unroll
+    for (int q = 0; q < S; ++q) {
+      const int i = 32 * q + lane;
+      const uint32_t id = i < nc ? list[i] : 0u;
+      v[q] = i < nc ? rel[id] : kRelCap;
+      col[q] = rows + (id >> 5);
+      bit[q] = 1u << (id & 31);
+      off[q] = tri_off(id);
+      crow[q] = ccol[q] = 0;
+    }
+    for (int g = 1; g < nc; ++g) {
+      const uint32_t o = of(off, g);
+      bool has[S];
+#pragma unroll
+      for (int q = 0; q < S; ++q) {
+        has[q] = 32 * q + lane < g && (col[q][o] & bit[q]);
+        if (has[q]) ccol[q] |= (M)1 << g;
+      }
+      const M m = mask_of(has);
+#pragma unroll
+      for (int q = 0; q < S; ++q)
+        if (32 * q + lane == g) crow[q] = m;
+    }
+  }
+
+  __device__ __forceinline__ uint32_t pairs(M P, uint32_t c) {
+    const uint32_t lt = lanemask_lt();
+    uint32_t tot[S], R[S], mine = 0;
+    bool act[S];
+#pragma unroll
+    for (int q = 0; q < S; ++q) {
+      const bool here = in(P, q);
+      tot[q] = here ? (uint32_t)pop(crow[q] & P) : 0u;
+      R[q] = here ? (uint32_t)pop(ccol[q] & P) + tot[q] : 0u;
+      act[q] = tot[q] != 0;
+      mine += tot[q];
+    }
+    const uint32_t sum = __reduce_add_sync(KCL_FULL, mine);
+    if (sum == 0) return c;
+    bool low[S], amb = false;
+#pragma unroll
+    for (int q = 0; q < S; ++q) {
+      low[q] = R[q] != 0 && v[q] + R[q] < c;
+      amb |= R[q] != 0 && !low[q] && v[q] < c + sum;
+    }
+    if (!__any_sync(KCL_FULL, amb)) {
+      const M Lg = mask_of(low);
+      if (!Lg) return c + sum;
+      uint32_t inc[S], taken = 0;
+#pragma unroll
+      for (int q = 0; q < S; ++q) {
+        inc[q] = low[q] ? (uint32_t)pop(ccol[q] & P & ~Lg) : 0u;
+        taken += inc[q];
+      }
+      bool clash = false;
+      for (M rem = Lg & mask_of(act); rem; rem &= rem - 1) {
+        const int u = first(rem);
+        const uint32_t vu = of(v, u), ru = of(R, u);
+        bool take[S];
+#pragma unroll
+        for (int q = 0; q < S; ++q) {
+          const bool has = low[q] && ((ccol[q] >> u) & 1u);
+          take[q] = has && v[q] + R[q] < vu;
+          clash |= has && !take[q] && v[q] < vu + ru;
+          inc[q] += take[q];
+        }
+        const uint32_t n = (uint32_t)pop(mask_of(take));
+#pragma unroll
+        for (int q = 0; q < S; ++q)
+          if (32 * q + lane == u) inc[q] += tot[q] - n;
+      }
+      if (!__any_sync(KCL_FULL, clash)) {
+        uint32_t fell = 0u - taken;
+#pragma unroll
+        for (int q = 0; q < S; ++q) {
+          v[q] += inc[q];
+          if (!low[q]) fell += tot[q];
+        }
+        return c + __reduce_add_sync(KCL_FULL, fell);
+      }
+    }
+    for (M rem = mask_of(act); rem; rem &= rem - 1) {
+      const int u = first(rem);
+      const M V = P & of(crow, u);
+      const uint32_t vu = of(v, u);
+      const bool own = vu < c;  // strict: ties stay with the earlier argmin
+      const uint32_t c0 = own ? vu : c;
+      uint32_t c1 = c0;
+#pragma unroll
+      for (int q = 0; q < S; ++q) {
+        const uint32_t vm = S == 1 ? (uint32_t)V : (uint32_t)(V >> (32 * q));
+        if (S == 1 || vm) {
+          const uint32_t m = word_fixed_point((vm >> lane) & 1u ? (int)(v[q] - c1) : -1, lt);
+          v[q] += ((vm & ~m) >> lane) & 1u;
+          c1 += (uint32_t)__popc(m);
+        }
+      }
+      if (own) {
+#pragma unroll
+        for (int q = 0; q < S; ++q)
+          if (32 * q + lane == u) v[q] += c1 - c0;
+      } else {
+        c = c1;
+      }
+    }
+    return c;
+  }
+
+  // Level L of the stream over P (kCDensestNoAtom.c:218-267).
+  template <int L>
+  __device__ __forceinline__ uint32_t level(M P, uint32_t c) {
+    if constexpr (L == 2) {
+      return pairs(P, c);
+    } else {
+      for (M rem = P; rem; rem &= rem - 1) {
+        const int u = first(rem);
+        const M Q = P & of(crow, u);
+        if (pop(Q) < L - 1) continue;
+        const uint32_t vu = of(v, u);
+        const bool own = vu < c;
+        const uint32_t c0 = own ? vu : c;
+        const uint32_t c1 = level<L - 1>(Q, c0);
+        if (own) {
+#pragma unroll
+          for (int q = 0; q < S; ++q)
+            if (32 * q + lane == u) v[q] += c1 - c0;
+        } else {
+          c = c1;
+        }
+      }
+      return c;
+    }
+  }
+
+  template <int K>
+  __device__ __forceinline__ uint32_t run(const uint32_t *rows, const uint16_t *list, int nc, const uint32_t *rel,
+                                          unsigned long long *acc, uint32_t c) {
+    load(rows, list, nc, rel);
+    c = level<K - 2>(nc == 32 * S ? ~(M)0 : ((M)1 << nc) - 1, c);
+#pragma unroll
+    for (int q = 0; q < S; ++q) {
+      const int i = 32 * q + lane;
+      if (i < nc) {
+        const uint32_t id = list[i], d = v[q] - rel[id];
+        if (d) atomicAdd(acc + id, (unsigned long long)d);
+      }
+    }
+    return c;
+  }
+};
+
+// The members of P (lane w: word w), ascending, into list.
+__device__ __forceinline__ int list_members(uint32_t P, uint16_t *list, int lane) {
+  const uint32_t lt = lanemask_lt();
+  int np = 0;
+  uint32_t nz = __ballot_sync(KCL_FULL, P != 0);
+  while (nz) {
+    const int L = __ffs(nz) - 1;
+    nz &= nz - 1;
+    const uint32_t word = __shfl_sync(KCL_FULL, P, L);
+    if ((word >> lane) & 1u) list[np + __popc(word & lt)] = (uint16_t)((L << 5) | lane);
+    np += __popc(word);
+  }
+  return np;
+}
+
+// ACC: the values are the root's own (shared by its streams, read only) and
+// increments go to acc; else the values are the stream's and are updated.
+template <bool ACC>
+struct PairLevel {
+  const uint32_t *rows;     // the root's triangular rows
+  uint32_t *val;            // values by local id
+  unsigned long long *acc;  // ACC: the root's increments
+  uint32_t *scratch;        // pair_words(dmax) words, 16-byte aligned
+  int lane;
+
+  __device__ __forceinline__ uint32_t *pw() const { return scratch; }
+  __device__ __forceinline__ uint32_t *ro() const { return scratch + 32; }
+  __device__ __forceinline__ uint2 *sv() const { return reinterpret_cast<uint2 *>(scratch + 64); }
+  __device__ __forceinline__ uint32_t *vv() const { return scratch + 128; }
+  __device__ __forceinline__ uint8_t *ci() const { return reinterpret_cast<uint8_t *>(scratch + 128 + kPairMembers); }
+  __device__ __forceinline__ uint16_t *ilist() const {
+    return reinterpret_cast<uint16_t *>(scratch + 128 + kPairMembers + kPairMembers / 4);
+  }
+  __device__ __forceinline__ uint16_t *list() const { return ilist() + kPairMembers; }
+
+  // Lane g's row offset and tot: |P ∩ row(u)|.
+  __device__ __forceinline__ uint32_t tot_of(int j, int np, uint32_t &off) const {
+    uint32_t t = 0;
+    off = 0;
+    if (j < np) {
+      const uint32_t u = list()[j];
+      off = tri_off(u);
+      const uint32_t *r = rows + off, *p = pw();
+      const int hi = (int)(u >> 5);
+      for (int w = 0; w <= hi; ++w) t += (uint32_t)__popc(r[w] & p[w]);
+    }
+    return t;
+  }
+
+  __device__ __forceinline__ void put(uint32_t id, uint32_t v0, uint32_t v) const {
+    if constexpr (ACC) {
+      if (v != v0) atomicAdd(acc + id, (unsigned long long)(v - v0));
+    } else {
+      val[id] = v;
+    }
+  }
+
+  // Bits of T for the member of id (list position j): the group's rows, read
+  // word by word at its bit.  A row ends at its own word; what is read beyond
+  // belongs to ids above u and is masked off (only u's after i in P hold i).
+  __device__ __forceinline__ uint32_t column(uint32_t id, int j, int a, int ng) const {
+    const uint32_t *col = rows + (id >> 5);
+    const uint32_t bit = 1u << (id & 31);
+    uint32_t t = 0;
+    for (int g = 0; g < ng; g += 4) {
+      const uint4 o = *reinterpret_cast<const uint4 *>(ro() + g);
+      uint32_t x = 0;
+      if (col[o.x] & bit) x |= 1u;
+      if (col[o.y] & bit) x |= 2u;
+      if (col[o.z] & bit) x |= 4u;
+      if (col[o.w] & bit) x |= 8u;
+      t |= x << g;
+    }
+    const int lo = j + 1 - a;
+    const uint32_t gmask = ng < 32 ? (1u << ng) - 1u : 0xffffffffu;
+    return t & (lo <= 0 ? gmask : (lo >= 32 ? 0u : gmask & (0xffffffffu << lo)));
+  }
+
+  // A chain of one slot whose every candidate is in I with nothing between
+  // them: the takers among `has` from prefix value c (which grows by the rest).
+  __device__ __forceinline__ uint32_t takers_dense(bool has, uint32_t v, uint32_t &c, uint32_t lt) const {
+    const uint32_t vm = __ballot_sync(KCL_FULL, has);
+    if (!vm) return 0;
+    const uint32_t m = word_fixed_point(has ? (int)(v - c) : -1, lt);
+    c += (uint32_t)__popc(m);
+    return vm & ~m;
+  }
+  // The same when members outside I stand between them: `ahead` members of V
+  // come before this lane's, of which `taken` took their clique in earlier
+  // slots; a candidate takes iff its value is below c + ahead - (takers before).
+  __device__ __forceinline__ uint32_t takers_sparse(bool has, uint32_t v, uint32_t c, uint32_t ahead, uint32_t taken,
+                                                    uint32_t lt) const {
+    const int z = has ? (int)(ahead + c - v - taken) : 0;
+    uint32_t mk = __ballot_sync(KCL_FULL, z > 0);
+    if (mk) {
+      for (int it = 0; it < 33; ++it) {
+        const uint32_t m2 = __ballot_sync(KCL_FULL, z > __popc(mk & lt));
+        if (m2 == mk) break;
+        mk = m2;
+      }
+    }
+    return mk;
+  }
+  // V's words (lane = word) and the members of V in the words before it.
+  __device__ __forceinline__ void words_of(uint32_t u, uint32_t off, uint32_t &Q, uint32_t &pre) const {
+    Q = lane <= (int)(u >> 5) ? rows[off + lane] & pw()[lane] : 0u;
+    const uint32_t own = (uint32_t)__popc(Q);
+    pre = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(KCL_FULL, pre, o);
+      if (lane >= o) pre += y;
+    }
+    pre -= own;
+  }
+  __device__ __forceinline__ uint32_t ahead_of(uint32_t id, uint32_t Q, uint32_t pre) const {
+    const uint32_t w = __shfl_sync(KCL_FULL, Q, id >> 5), p = __shfl_sync(KCL_FULL, pre, id >> 5);
+    return p + (uint32_t)__popc(w & ((1u << (id & 31)) - 1u));
+  }
+
+  // At most one slot: values in registers.  ALL: I is all of P (<= 32).
+  template <bool ALL>
+  __device__ __forceinline__ uint32_t run1(int np, int ni, uint32_t c) const {
+    const uint32_t lt = lanemask_lt();
+    const int at = lane < ni ? (ALL ? lane : (int)ilist()[lane]) : -1;
+    const uint32_t id = at >= 0 ? list()[at] : 0u;
+    const uint32_t v0 = at >= 0 ? val[id] : 0x7fffffffu;
+    uint32_t v = v0;
+    for (int a = 0; a < np; a += 32) {
+      const int ng = np - a < 32 ? np - a : 32;
+      uint32_t off;
+      const uint32_t tot = tot_of(a + lane, np, off);
+      const uint32_t sum = __reduce_add_sync(KCL_FULL, tot);
+      if (sum == 0) continue;
+      const int gi = at - a;
+      const bool live = at >= 0 && gi < ng, in = live && gi >= 0;
+      const uint32_t ti = __shfl_sync(KCL_FULL, tot, gi & 31);
+      const uint32_t S = 32u + (in ? ti : 0u);
+      const bool low = live && v + S < c;
+      if (!__any_sync(KCL_FULL, live && !low && v < c + sum)) {
+        if (!__any_sync(KCL_FULL, low)) {
+          c += sum;
+          continue;
+        }
+        const uint32_t Lg = __reduce_or_sync(KCL_FULL, in && low ? 1u << gi : 0u);
+        __syncwarp();
+        ro()[lane] = off;
+        if (in && low) sv()[gi] = make_uint2(v, S);
+        __syncwarp();
+        uint32_t T = column(id, at, a, ng);
+        if (!low) T = 0;  // the others always fall
+        uint32_t inc = (uint32_t)__popc(T & ~Lg);
+        const uint32_t taken = inc;
+        bool clash = false;
+        for (uint32_t rem = Lg; rem; rem &= rem - 1) {
+          const int g = __ffs(rem) - 1;
+          const uint2 x = sv()[g];
+          const bool has = (T >> g) & 1u, take = has && v + S < x.x;
+          clash |= has && !take && v < x.x + x.y;
+          const uint32_t n = (uint32_t)__popc(__ballot_sync(KCL_FULL, take));
+          inc += take;
+          if (in && gi == g) inc += ti - n;
+        }
+        if (!__any_sync(KCL_FULL, clash)) {
+          v += inc;
+          c += __reduce_add_sync(KCL_FULL, (((Lg >> lane) & 1u) ? 0u : tot) - taken);
+          continue;
+        }
+      }
+      const uint32_t *col = rows + (id >> 5);
+      const uint32_t bit = 1u << (id & 31);
+      for (uint32_t rem = __ballot_sync(KCL_FULL, tot != 0); rem; rem &= rem - 1) {
+        const int g = __ffs(rem) - 1;
+        const uint32_t og = __shfl_sync(KCL_FULL, off, g);
+        const bool has = at >= 0 && gi < g && (col[og] & bit);
+        uint32_t vu = 0x7fffffffu;
+        if constexpr (ALL) {
+          vu = __shfl_sync(KCL_FULL, v, g);
+        } else {
+          const uint32_t who = __ballot_sync(KCL_FULL, in && gi == g);
+          if (who) vu = __shfl_sync(KCL_FULL, v, __ffs(who) - 1);
+        }
+        const bool own = vu < c;  // strict: ties stay with the earlier argmin
+        const uint32_t c0 = own ? vu : c;
+        uint32_t fell, mk;
+        if constexpr (ALL) {
+          uint32_t cl = c0;
+          mk = takers_dense(has, v, cl, lt);
+          fell = cl - c0;
+        } else {
+          const uint32_t tu = __shfl_sync(KCL_FULL, tot, g);
+          const uint32_t x = v - c0;
+          if (!__any_sync(KCL_FULL, has && x < tu)) {
+            mk = __ballot_sync(KCL_FULL, has && (int)x < 0);
+          } else {
+            uint32_t Q, pre;
+            words_of(list()[a + g], og, Q, pre);
+            mk = takers_sparse(has, v, c0, ahead_of(id, Q, pre), 0u, lt);
+          }
+          fell = tu - (uint32_t)__popc(mk);
+        }
+        v += (mk >> lane) & 1u;
+        if (!own) c += fell;
+        else if (in && gi == g) v += fell;
+      }
+    }
+    if (at >= 0) put(id, v0, v);
+    __syncwarp();
+    return c;
+  }
+
+  // Several slots: values, increments and positions in the scratch, member
+  // 32 q + lane of I always handled by this lane.
+  __device__ __forceinline__ uint32_t run_slots(int np, int ni, uint32_t c) const {
+    const uint32_t lt = lanemask_lt();
+    const bool dense = ni == np;
+    uint32_t *const V = vv();
+    uint8_t *const I8 = ci();
+    const uint16_t *const il = ilist();
+    for (int i = lane; i < ni; i += 32) V[i] = val[list()[il[i]]];
+    for (int a = 0; a < np; a += 32) {
+      const int ng = np - a < 32 ? np - a : 32;
+      uint32_t off;
+      const uint32_t tot = tot_of(a + lane, np, off);
+      const uint32_t sum = __reduce_add_sync(KCL_FULL, tot);
+      if (sum == 0) continue;
+      int ns = 0;  // slots with a member at or before the group's last
+      while (32 * ns < ni && (int)il[32 * ns] < a + ng) ++ns;
+      uint32_t Lg = 0, Ig = 0;
+      bool amb = false, lows = false;
+      __syncwarp();
+      ro()[lane] = off;
+      for (int q = 0; q < ns; ++q) {
+        const int i = 32 * q + lane;
+        const int gi = i < ni ? (int)il[i] - a : 64;
+        const bool live = gi < ng, in = live && gi >= 0;
+        const uint32_t ti = __shfl_sync(KCL_FULL, tot, gi & 31);
+        if (live) {
+          const uint32_t v = V[i], S = 32u + (in ? ti : 0u);
+          const bool low = v + S < c;
+          lows |= low;
+          amb |= !low && v < c + sum;
+          if (in) {
+            sv()[gi] = low ? make_uint2(v, S) : make_uint2(0u, (uint32_t)i);
+            Ig |= 1u << gi;
+            if (low) Lg |= 1u << gi;
+          }
+        }
+      }
+      __syncwarp();
+      if (!__any_sync(KCL_FULL, amb)) {
+        if (!__any_sync(KCL_FULL, lows)) {
+          c += sum;
+          continue;
+        }
+        Lg = __reduce_or_sync(KCL_FULL, Lg);
+        uint32_t ng_taken = 0, taken = 0;  // lane g: takers of u_g's chain, u_g in L
+        bool clash = false;
+        for (int q = 0; q < ns; ++q) {
+          const int i = 32 * q + lane;
+          const int j = i < ni ? (int)il[i] : a + 64;
+          const bool in = j >= a && j < a + ng;
+          const uint32_t ti = __shfl_sync(KCL_FULL, tot, j & 31);
+          const uint32_t v = i < ni ? V[i] : 0x7fffffffu, S = 32u + (in ? ti : 0u);
+          const bool low = j < a + ng && v + S < c;
+          uint32_t inc = 0;
+          if (__any_sync(KCL_FULL, low)) {
+            uint32_t T = column(i < ni ? list()[j] : 0u, j, a, ng);
+            if (!low) T = 0;  // the others always fall
+            inc = (uint32_t)__popc(T & ~Lg);
+            taken += inc;
+            for (uint32_t rem = Lg; rem; rem &= rem - 1) {
+              const int g = __ffs(rem) - 1;
+              const uint2 x = sv()[g];
+              const bool has = (T >> g) & 1u, take = has && v + S < x.x;
+              clash |= has && !take && v < x.x + x.y;
+              const uint32_t n = (uint32_t)__popc(__ballot_sync(KCL_FULL, take));
+              if (lane == g) ng_taken += n;
+              inc += take;
+            }
+          }
+          if (i < ni) I8[i] = (uint8_t)inc;
+        }
+        if (!__any_sync(KCL_FULL, clash)) {
+          const uint32_t fell = ((Lg >> lane) & 1u) ? tot - ng_taken : 0u;
+          for (int q = 0; q < ns; ++q) {
+            const int i = 32 * q + lane;
+            const int gi = i < ni ? (int)il[i] - a : 64;
+            const uint32_t f = __shfl_sync(KCL_FULL, fell, gi & 31);
+            if (i < ni) V[i] += I8[i] + (gi >= 0 && gi < ng ? f : 0u);
+          }
+          c += __reduce_add_sync(KCL_FULL, (((Lg >> lane) & 1u) ? 0u : tot) - taken);
+          continue;
+        }
+        // the chains need the members' places, not their values
+        __syncwarp();
+        for (int q = 0; q < ns; ++q) {
+          const int i = 32 * q + lane;
+          const int gi = i < ni ? (int)il[i] - a : 64;
+          if (gi >= 0 && gi < ng) sv()[gi].y = (uint32_t)i;
+        }
+        __syncwarp();
+      } else if (__any_sync(KCL_FULL, Lg != 0)) {
+        for (int q = 0; q < ns; ++q) {
+          const int i = 32 * q + lane;
+          const int gi = i < ni ? (int)il[i] - a : 64;
+          if (gi >= 0 && gi < ng) sv()[gi].y = (uint32_t)i;
+        }
+        __syncwarp();
+      }
+      Ig = __reduce_or_sync(KCL_FULL, Ig);
+      for (uint32_t rem = __ballot_sync(KCL_FULL, tot != 0); rem; rem &= rem - 1) {
+        const int g = __ffs(rem) - 1;
+        const uint32_t og = ro()[g];
+        const uint32_t tu = __shfl_sync(KCL_FULL, tot, g);
+        uint32_t vu = 0x7fffffffu, iu = 0;
+        if ((Ig >> g) & 1u) {
+          iu = sv()[g].y;
+          __syncwarp();  // the value is its own lane's
+          vu = V[iu];
+        }
+        const bool own = vu < c;  // strict: ties stay with the earlier argmin
+        const uint32_t c0 = own ? vu : c;
+        uint32_t n = 0;  // takers
+        if (dense) {
+          uint32_t cl = c0;
+          for (int i0 = 0; i0 < a + g; i0 += 32) {
+            const int i = i0 + lane;
+            bool has = false;
+            uint32_t v = 0;
+            if (i < a + g) {
+              const uint32_t id = list()[i];
+              has = (rows[og + (id >> 5)] >> (id & 31)) & 1u;
+              v = V[i];
+            }
+            if ((takers_dense(has, v, cl, lt) >> lane) & 1u) V[i] = v + 1u;
+          }
+          n = tu - (cl - c0);
+        } else {
+          bool near = false;
+          uint32_t hasq = 0;
+          for (int q = 0; q < ns; ++q) {
+            const int i = 32 * q + lane;
+            const int j = i < ni ? (int)il[i] : a + 64;
+            if (j < a + g) {
+              const uint32_t id = list()[j];
+              if ((rows[og + (id >> 5)] >> (id & 31)) & 1u) {
+                hasq |= 1u << q;
+                near |= V[i] - c0 < tu;
+              }
+            }
+          }
+          if (!__any_sync(KCL_FULL, near)) {
+            for (int q = 0; q < ns; ++q)
+              if ((hasq >> q) & 1u) {
+                const int i = 32 * q + lane;
+                const uint32_t v = V[i], t = (v - c0) >> 31;
+                V[i] = v + t;
+                n += t;
+              }
+            n = __reduce_add_sync(KCL_FULL, n);
+          } else {
+            uint32_t Q, pre;
+            words_of(list()[a + g], og, Q, pre);
+            for (int q = 0; q < ns; ++q) {
+              const int i = 32 * q + lane;
+              const bool has = (hasq >> q) & 1u;
+              const uint32_t id = has ? list()[il[i]] : 0u;
+              const uint32_t v = has ? V[i] : 0u;
+              const uint32_t mk = takers_sparse(has, v, c0, ahead_of(id, Q, pre), n, lt);
+              if ((mk >> lane) & 1u) V[i] = v + 1u;
+              n += (uint32_t)__popc(mk);
+            }
+          }
+        }
+        const uint32_t fell = tu - n;
+        if (!own) c += fell;
+        else if (lane == (int)(iu & 31u)) V[iu] += fell;
+      }
+    }
+    for (int i = lane; i < ni; i += 32) {
+      const uint32_t id = list()[il[i]];
+      put(id, ACC ? val[id] : 0u, V[i]);
+    }
+    __syncwarp();
+    return c;
+  }
+
+  // The two levels over P (lane w: word w) from prefix value c.  Returns
+  // false, with nothing changed, when I outgrows the scratch.
+  __device__ __forceinline__ bool operator()(uint32_t P, uint32_t &c) const {
+    const uint32_t lt = lanemask_lt();
+    __syncwarp();
+    pw()[lane] = P;
+    const int np = list_members(P, list(), lane);
+    if (np < 2) return true;
+    __syncwarp();
+    if (np <= 32) {  // one slot holds P: choosing I would cost more than it saves
+      c = run1<true>(np, np, c);
+      return true;
+    }
+    const uint32_t reach = c + (uint32_t)np * (uint32_t)(np - 1) / 2u;
+    int ni = 0;
+    for (int b = 0; b < np; b += 32) {
+      const bool in = b + lane < np && val[list()[b + lane]] < reach;
+      const uint32_t mk = __ballot_sync(KCL_FULL, in);
+      const int p = ni + __popc(mk & lt);
+      if (in && p < kPairMembers) ilist()[p] = (uint16_t)(b + lane);
+      ni += __popc(mk);
+    }
+    if (ni <= 32) {
+      __syncwarp();
+      c = run1<false>(np, ni, c);
+      return true;
+    }
+    if (2 * ni > np && np <= kPairMembers) {  // then I = P: no members between
+      for (int i = lane; i < np; i += 32) ilist()[i] = (uint16_t)i;
+      ni = np;
+    }
+    if (ni > kPairMembers) return false;
+    __syncwarp();
+    c = run_slots(np, ni, c);
+    return true;
+  }
+};
+
 // Level L of a root-edge stream over candidates P with prefix argmin g of
 // current value cg (kCDensestNoAtom.c:173-188 for L = 2, 237-259 above).
 // Returns g's new value; the argmin of a deeper prefix, when it is u, is
 // written back by u's lane.  SKIP (one word per lane, 32-bit values): the
-// last level runs chain_word1 with lo, the per-word lower bounds.
-template <int L, int WPL, typename VA, bool SKIP>
+// last level runs chain_word1 with lo, the per-word lower bounds.  PAIR (the
+// same, private values): the last two levels run as one PairLevel, and one
+// word at a time only when that has no room (pair: its scratch).
+template <int L, int WPL, typename VA, bool SKIP, bool PAIR = false>
 __device__ __forceinline__ typename VA::T seq_rec(const Bits<WPL> &P, typename VA::T cg, const uint32_t *rows,
-                                                  const VA &va, typename VA::T lo, int lane, uint32_t *err) {
+                                                  const VA &va, typename VA::T lo, int lane, uint32_t *err,
+                                                  uint32_t *pair = nullptr) {
   using T = typename VA::T;
-  if constexpr (L == 1) {
+  if constexpr (PAIR && L == 2) {
+    static_assert(WPL == 1 && SKIP, "the pair level needs one word per lane and 32-bit values");
+    if (PairLevel<false>{rows, va.cur, nullptr, pair, lane}(P.w[0], cg)) return cg;
+    lo = 0xffffffffu;
+    uint32_t nz = __ballot_sync(KCL_FULL, P.w[0] != 0);
+    while (nz) {
+      const int w = __ffs(nz) - 1;
+      nz &= nz - 1;
+      const uint32_t word = __shfl_sync(KCL_FULL, P.w[0], w);
+      const uint32_t val = __reduce_min_sync(KCL_FULL, ((word >> lane) & 1u) ? va.cur[(w << 5) | lane] : 0xffffffffu);
+      if (lane == w) lo = val;
+    }
+    return seq_rec<2, 1, VA, true, false>(P, cg, rows, va, lo, lane, err);
+  } else if constexpr (L == 1) {
     if constexpr (SKIP) {
       static_assert(WPL == 1 && sizeof(T) == 4, "the word skip needs one word per lane and 32-bit values");
       return chain_word1<VA>(P.w[0], cg, va, lo, lane, err);
@@ -734,7 +1415,7 @@ __device__ __forceinline__ typename VA::T seq_rec(const Bits<WPL> &P, typename V
         Bits<1> Q;
         Q.w[0] = in_row ? (P.w[0] & row0[(uint32_t)b * stride]) : 0u;
         const T c0 = take ? vu : cg;
-        const T c1 = seq_rec<L - 1, 1, VA, SKIP>(Q, c0, rows, va, lo, lane, err);
+        const T c1 = seq_rec<L - 1, 1, VA, SKIP, PAIR>(Q, c0, rows, va, lo, lane, err, pair);
         if (take) {
           if (lane == b) va.add(u, c1 - c0, err);
         } else {
@@ -783,6 +1464,12 @@ __device__ __forceinline__ void for_members(const Bits<WPL> &C, int lane, F &&f)
 // the root's shared counter (largest candidate sets first); increments go to
 // the CTA's acc[] (kCDensestNoAtom.c:270-295 per root edge).
 //
+// k >= 4, rows in shared memory: the streams read rel, the root's values as
+// 32-bit offsets from the smallest of them capped at kRelCap; a stream whose
+// prefix value cannot reach the cap uses them (a capped member then lies above
+// every prefix value, so the cap changes no comparison).  Otherwise the
+// stream makes its own values:
+//
 // A stream's values fit the 32-bit form when, with off = the smallest
 // pass-start value among {s, t} and C and cap = (the edge argmin's value
 // - off) + the most increments one vertex can take in the stream + 64, cap
@@ -793,7 +1480,8 @@ __device__ __forceinline__ void for_members(const Bits<WPL> &C, int lane, F &&f)
 template <int K, int WPL>
 __device__ __forceinline__ void seq_streams(uint32_t *next, int d, const uint32_t *rows,
                                             const unsigned long long *base, uint32_t *cur,
-                                            unsigned long long *acc, int lane, uint32_t *err) {
+                                            unsigned long long *acc, const uint32_t *rel, uint32_t *pair, int lane,
+                                            uint32_t *err) {
   for (;;) {
     int q = 0;
     if (lane == 0) q = (int)atomicAdd(next, 1u);
@@ -803,6 +1491,57 @@ __device__ __forceinline__ void seq_streams(uint32_t *next, int d, const uint32_
     const Bits<WPL> C = load_row<WPL, true>(rows, j, 0, lane);
     if (!any_bits<WPL>(C)) continue;
     const int g0 = base[j] < base[d] ? j : d;  // kCDensestNoAtom.c:287
+    if constexpr (K >= 4 && WPL == 1) {
+      // The root's 32-bit values serve the stream when no prefix value it can
+      // reach comes near their cap (see kRelCap).
+      const uint32_t nc = __reduce_add_sync(KCL_FULL, (uint32_t)__popc(C.w[0]));
+      if (nc < (uint32_t)(K - 2)) continue;
+      unsigned long long bound = 1;  // C(nc, K - 2): the stream's cliques at most
+#pragma unroll
+      for (uint32_t i = 0; i < (uint32_t)(K - 2); ++i) bound = bound * (nc - i) / (i + 1u);
+      const uint32_t c0 = rel[g0];
+      if (bound + 64 < (unsigned long long)(kRelCap - c0)) {
+        // Two slots cost 64 column reads per member up front: k = 4, with one
+        // pair of levels per stream, has nothing to spread them over.
+        constexpr int kTiny = K == 4 ? 32 : 64;
+        if (nc <= (uint32_t)kTiny) {
+          uint16_t *list = PairLevel<true>{nullptr, nullptr, nullptr, pair, lane}.list();
+          __syncwarp();
+          list_members(C.w[0], list, lane);
+          __syncwarp();
+          uint32_t c1;
+          if (K == 4 || nc <= 32) {
+            TinyStream<1> ts;
+            ts.lane = lane;
+            c1 = ts.template run<K>(rows, list, (int)nc, rel, acc, c0);
+          } else {
+            TinyStream<2> ts;
+            ts.lane = lane;
+            c1 = ts.template run<K>(rows, list, (int)nc, rel, acc, c0);
+          }
+          if (lane == 0 && c1 != c0) atomicAdd(&acc[g0], (unsigned long long)(c1 - c0));
+          continue;
+        }
+        if constexpr (K == 4) {
+          uint32_t c = c0;
+          if (PairLevel<true>{rows, const_cast<uint32_t *>(rel), acc, pair, lane}(C.w[0], c)) {
+            if (lane == 0 && c != c0) atomicAdd(&acc[g0], (unsigned long long)(c - c0));
+            continue;
+          }
+        } else {
+          for_members<1>(C, lane, [&](int i) { cur[i] = rel[i]; });
+          const Vals32 va{cur};
+          const uint32_t c1 = seq_rec<K - 2, 1, Vals32, true, true>(C, c0, rows, va, 0u, lane, err, pair);
+          __syncwarp();
+          for_members<1>(C, lane, [&](int i) {
+            const uint32_t delta = cur[i] - rel[i];
+            if (delta) atomicAdd(&acc[i], (unsigned long long)delta);
+          });
+          if (lane == 0 && c1 != c0) atomicAdd(&acc[g0], (unsigned long long)(c1 - c0));
+          continue;
+        }
+      }
+    }
     bool r32 = false;
     unsigned long long off = 0, cap = 0;
     if constexpr (K <= 5) {
@@ -976,7 +1715,7 @@ __device__ __forceinline__ uint32_t find_victim(const PassArgs &a, int need, int
 // and <= 42 at k = 5 with 24-warp CTAs), one for the deeper ones, which would
 // otherwise spill.
 template <int MODE, int K>
-constexpr int min_ctas_m() { return K <= (MODE == MODE_SEQ ? 4 : 5) ? 2 : 1; }
+constexpr int min_ctas_m() { return MODE == MODE_SEQ || K <= 5 ? 2 : 1; }
 
 template <int MODE, int K, int WPL, bool ROWS_IN_SMEM, bool IDENT = false>
 __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()) tier_m_kernel(PassArgs a) {
@@ -992,13 +1731,15 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
   unsigned long long *acc = reinterpret_cast<unsigned long long *>(smem_raw + lay.acc);
   uint16_t *rank = reinterpret_cast<uint16_t *>(smem_raw + lay.rank);
   uint16_t *inv = reinterpret_cast<uint16_t *>(smem_raw + lay.inv);
-  uint32_t *dl = reinterpret_cast<uint32_t *>(smem_raw + lay.dl) + (size_t)wid * (dmax + 1);
+  uint32_t *dl = reinterpret_cast<uint32_t *>(smem_raw + lay.dl) + (size_t)wid * seq_warp_words(K, a.dmax, ROWS_IN_SMEM);
+  uint32_t *pair = K == 4 ? dl : dl + ((size_t)dmax + 4) / 4 * 4;
+  uint32_t *rel = reinterpret_cast<uint32_t *>(smem_raw + lay.rel);
   uint32_t *cbuf = reinterpret_cast<uint32_t *>(smem_raw + lay.cbuf) + (size_t)wid * cbuf_words(a.dmax);
 
   __shared__ uint32_t s_idx;
   __shared__ int s_tau;
   __shared__ unsigned long long s_sum;
-  __shared__ unsigned long long s_off;  // shared-load Seq: the root's smallest value
+  __shared__ unsigned long long s_off;  // Seq: the root's smallest value
 
   if constexpr (MODE == MODE_SEQ) {
     for (int i = tid; i <= dmax; i += NW * 32) acc[i] = 0;
@@ -1081,8 +1822,22 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
           cur[i] = v < kSharedCap ? (uint32_t)v : kSharedCap;
         }
       } else {
-        for (int i = tid; i < d; i += NW * 32) base[i] = a.r_in[a.cols[o + i]];
-        if (tid == 0) base[d] = a.r_in[s];
+        unsigned long long mn = ~0ull;
+        for (int i = tid; i <= d; i += NW * 32) {
+          const unsigned long long v = a.r_in[i < d ? a.cols[o + i] : s];
+          base[i] = v;
+          mn = v < mn ? v : mn;
+        }
+        if constexpr (K >= 4 && ROWS_IN_SMEM) {
+          mn = warp_min_u64(mn);
+          if (lane == 0) atomicMin(&s_off, mn);
+          __syncthreads();
+          const unsigned long long off = s_off;
+          for (int i = tid; i <= d; i += NW * 32) {
+            const unsigned long long v = base[i] - off;
+            rel[i] = v < kRelCap ? (uint32_t)v : kRelCap;
+          }
+        }
       }
     }
     __syncthreads();
@@ -1136,7 +1891,7 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
         seq_streams_shared<K, WPL>(next, d, rows, list, s, a.out, s_off, reinterpret_cast<uint32_t *>(acc), dl,
                                    lane, a.err);
       else
-        seq_streams<K, WPL>(next, d, rows, base, dl, acc, lane, a.err);
+        seq_streams<K, WPL>(next, d, rows, base, dl, acc, rel, pair, lane, a.err);
       __syncthreads();
       for (int i = tid; i <= d; i += NW * 32) {
         const unsigned long long v = acc[i];
@@ -1277,15 +2032,18 @@ static cudaError_t pick_warps(Fn fn, LaunchCache &lc, uint32_t dmax, bool rows_i
   }
   int best = 0, best_warps = -1;
   for (int w = lo; w <= hi; w = w < 8 ? w * 2 : w + step) {
-    if (req > 0 && w != req) continue;
     const size_t sm = layout_m(MODE, K, dmax, w, rows_in_smem).total;
     if (sm > 227 * 1024) continue;
+    if (req > 0) {  // the requested width, or the widest below it that fits
+      if (w <= req) best = w;
+      continue;
+    }
     int per_sm = 0;
     cudaError_t e = prepare(fn, lc, w * 32, sm, &per_sm);
     if (e != cudaSuccess) return e;
     if (per_sm * w > best_warps) { best_warps = per_sm * w; best = w; }
   }
-  if (best == 0) best = req > hi ? hi : lo;  // a width this launch cannot take: the nearest one
+  if (best == 0) best = lo;
   std::lock_guard<std::mutex> g(lc.mu);
   if (lc.nnw < 32) {
     lc.nw_dev[lc.nnw] = dev;
@@ -1356,19 +2114,16 @@ cudaError_t launch_tier(const TierLaunch &t, dev::PassArgs a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-template <int MODE>
+// The kernels of MODE for k in [LO, HI].
+template <int MODE, int LO = 2, int HI = 8>
 cudaError_t launch_mode(int k, const TierLaunch &t, dev::PassArgs a, cudaStream_t st) {
-  switch (k) {
-    case 2: if constexpr (MODE == dev::MODE_ORDER) return launch_tier<MODE, 2>(t, a, st); else break;
-    case 3: return launch_tier<MODE, 3>(t, a, st);
-    case 4: return launch_tier<MODE, 4>(t, a, st);
-    case 5: return launch_tier<MODE, 5>(t, a, st);
-    case 6: return launch_tier<MODE, 6>(t, a, st);
-    case 7: return launch_tier<MODE, 7>(t, a, st);
-    case 8: return launch_tier<MODE, 8>(t, a, st);
-    default: break;
+  if constexpr (LO > HI) {
+    return cudaErrorInvalidValue;
+  } else if constexpr (LO < 3 && MODE != dev::MODE_ORDER) {
+    return launch_mode<MODE, 3, HI>(k, t, a, st);
+  } else {
+    return k == LO ? launch_tier<MODE, LO>(t, a, st) : launch_mode<MODE, LO + 1, HI>(k, t, a, st);
   }
-  return cudaErrorInvalidValue;
 }
 
 }  // namespace kclpp
