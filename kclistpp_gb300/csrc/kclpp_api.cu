@@ -91,6 +91,8 @@ struct kclpp_graph {
   uint64_t *d_off = nullptr;
   uint32_t *d_cols = nullptr;
   uint32_t *d_src = nullptr;
+  uint4 *d_bit_rows = nullptr;  // bitmap rows (PassArgs.bit_rows), or nullptr
+  uint32_t *d_bits = nullptr;
   uint32_t *d_roots = nullptr;
   // Two schedules over the same roots: [0] for the counting kernels (tier S up
   // to out-degree 64), [1] for the Seq kernel (tier S up to 16).
@@ -142,6 +144,20 @@ __global__ void k_count_edges(const uint32_t *src, const uint32_t *cols, uint64_
     c += (level[src[e]] < nstar && level[cols[e]] < nstar);
   c = dev::warp_sum(c);
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
+}
+
+// Bitmap rows: a warp per vertex that has one.
+__global__ void k_bit_rows(const uint64_t *off, const uint32_t *cols, const uint4 *rows, uint32_t *bits, uint32_t n) {
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  for (uint32_t v = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); v < n; v += warps) {
+    const uint4 r = rows[v];
+    if (r.x == 0xffffffffu) continue;
+    const uint64_t end = off[v + 1];
+    for (uint64_t e = off[v] + (threadIdx.x & 31); e < end; e += 32) {
+      const uint32_t t = cols[e] - r.y;
+      atomicOr(bits + r.x + (t >> 5), 1u << (t & 31));
+    }
+  }
 }
 
 inline int blocks_for(uint64_t n, int t = 256) { return (int)std::max<uint64_t>(1, (n + t - 1) / t); }
@@ -315,6 +331,38 @@ static kclpp_status build_schedule(kclpp_ctx *c, kclpp_graph *g) {
   return KCLPP_OK;
 }
 
+// Bitmap rows for the vertices whose out-list fills at least a bit in 64 of the
+// id range it spans (two words per edge): inducing a root's rows asks such a
+// vertex about 32 members at a time, where walking its list costs a look-up per
+// edge and mostly misses.  At most 8 bytes per edge; sparser lists stay short
+// for the ids they span and are walked.  Needs d_off and d_cols.
+static kclpp_status upload_bit_rows(kclpp_ctx *c, kclpp_graph *g) {
+  const HostDag &D = g->dag;
+  std::vector<uint4> rows(D.n);
+  uint64_t words = 0;
+  for (uint32_t v = 0; v < D.n; ++v) {
+    const uint64_t d = D.off[v + 1] - D.off[v];
+    rows[v] = make_uint4(0xffffffffu, 0u, 0u, 0u);
+    if (d < 2) continue;
+    const uint32_t lo = D.cols[D.off[v]], hi = D.cols[D.off[v + 1] - 1];
+    const uint64_t w = ((uint64_t)(hi - lo) >> 5) + 1;
+    if (w > 2 * d || words + w >= 0xffffffffull) continue;
+    rows[v] = make_uint4((uint32_t)words, lo, hi - lo + 1, 0u);
+    words += w;
+  }
+  if (!words) return KCLPP_OK;
+  KCL_TRY(dalloc(&g->d_bit_rows, D.n));
+  KCL_TRY(dalloc(&g->d_bits, words));
+  KCL_CUDA(cudaMemcpyAsync(g->d_bit_rows, rows.data(), (size_t)D.n * sizeof(uint4), cudaMemcpyHostToDevice, c->stream));
+  KCL_CUDA(cudaMemsetAsync(g->d_bits, 0, words * 4, c->stream));
+  k_bit_rows<<<std::min(blocks_for(D.n, 8), c->num_sms * 8), 256, 0, c->stream>>>(g->d_off, g->d_cols, g->d_bit_rows,
+                                                                                g->d_bits, D.n);
+  KCL_CUDA(cudaGetLastError());
+  KCL_CUDA(cudaStreamSynchronize(c->stream));
+  c->launches++;
+  return KCLPP_OK;
+}
+
 static kclpp_status upload_graph(kclpp_ctx *c, kclpp_graph *g) {
   const HostDag &D = g->dag;
   if (D.core > kTierLMax)
@@ -330,6 +378,7 @@ static kclpp_status upload_graph(kclpp_ctx *c, kclpp_graph *g) {
       for (uint64_t e = D.off[s]; e < D.off[s + 1]; ++e) src[e] = s;
     KCL_CUDA(cudaMemcpyAsync(g->d_src, src.data(), D.m() * 4, cudaMemcpyHostToDevice, c->stream));
     KCL_CUDA(cudaStreamSynchronize(c->stream));
+    KCL_TRY(upload_bit_rows(c, g));
   }
   KCL_TRY(build_schedule(c, g));
   const size_t n1 = (size_t)D.n + 1;
@@ -343,6 +392,7 @@ static kclpp_status upload_graph(kclpp_ctx *c, kclpp_graph *g) {
 }
 
 static void free_graph_dev(kclpp_graph *g) {
+  cudaFree(g->d_bit_rows); cudaFree(g->d_bits);
   cudaFree(g->d_off); cudaFree(g->d_cols); cudaFree(g->d_src); cudaFree(g->d_roots);
   cudaFree(g->d_a); cudaFree(g->d_b); cudaFree(g->d_rho); cudaFree(g->d_level);
   cudaFree(g->d_work); cudaFree(g->d_task); cudaFree(g->d_scalar); cudaFree(g->d_slab);
@@ -373,6 +423,8 @@ static kclpp_status run_tiers(kclpp_ctx *c, kclpp_graph *g, int mode, int k, dev
   a.err = c->d_err;
   a.slab = g->d_slab;
   a.slab_words = g->slab_words;
+  a.bit_rows = g->d_bit_rows;
+  a.bits = g->d_bits;
   // Root groups of one pass are independent (they read the pass-start vector
   // and add into the output), so they may run side by side: the later groups
   // fill the SMs that the first one's tail leaves idle.
@@ -1595,6 +1647,8 @@ kclpp_status ctx_check_err(kclpp_ctx *c) { return check_err(c); }
 const HostDag &graph_dag(const kclpp_graph *g) { return g->dag; }
 const uint64_t *graph_dev_offsets(const kclpp_graph *g) { return g->d_off; }
 const uint32_t *graph_dev_cols(const kclpp_graph *g) { return g->d_cols; }
+const uint4 *graph_dev_bit_rows(const kclpp_graph *g) { return g->d_bit_rows; }
+const uint32_t *graph_dev_bits(const kclpp_graph *g) { return g->d_bits; }
 int graph_device(const kclpp_graph *g) { return g->device; }
 }  // namespace kclpp
 

@@ -66,6 +66,11 @@ struct PassArgs {
   // of the pass, read by every stream when it starts and added to in place
   // when it closes.
   int shared_loads;
+  // Bitmap rows of the vertices whose out-lists are dense in their id range
+  // (nullptr: none): per vertex (first word in bits, id of its first bit, ids
+  // covered; first word 0xffffffff and 0 ids: no row).
+  const uint4 *bit_rows;
+  const uint32_t *bits;
 };
 
 // A root's member list: its DAG out-list, or its explicit list (peel recounts).
@@ -111,17 +116,6 @@ __device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v)
 __device__ __forceinline__ uint64_t vertex_key(const PassArgs &a, uint32_t v) {
   if (a.key_kind == KEY_SIM) return (uint64_t)__double_as_longlong(a.rho[v]);
   return (uint64_t)(0xFFFFFFFFu - a.level[v]);
-}
-
-// Lower bound of y in the ascending list[0, n).
-__device__ __forceinline__ int lower_bound_u32(const uint32_t *list, int n, uint32_t y) {
-  int lo = 0, hi = n;
-  while (lo < hi) {
-    int mid = (lo + hi) >> 1;
-    if (list[mid] < y) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
 }
 
 }  // namespace dev

@@ -9,6 +9,7 @@
 #include "../../include/kclpp.h"
 
 typedef struct CUstream_st *cudaStream_t;
+struct uint4;
 
 struct kclpp_edge_list {
   uint32_t n = 0;               // max id + 1 (ReadEdgeList semantics)
@@ -117,6 +118,8 @@ kclpp_status ctx_check_err(kclpp_ctx *c);
 const HostDag &graph_dag(const kclpp_graph *g);
 const uint64_t *graph_dev_offsets(const kclpp_graph *g);
 const uint32_t *graph_dev_cols(const kclpp_graph *g);
+const uint4 *graph_dev_bit_rows(const kclpp_graph *g);  // nullptr: none
+const uint32_t *graph_dev_bits(const kclpp_graph *g);
 int graph_device(const kclpp_graph *g);
 
 // Recounts of the k-clique core peel on the GPU (kclpp_peel.cu): for a batch

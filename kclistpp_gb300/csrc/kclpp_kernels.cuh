@@ -49,9 +49,58 @@ namespace dev {
 constexpr int kSMaxD = 64;
 constexpr int kSDl = kSMaxD + 1;  // per-lane delta stride
 
+// A root's members by id: an open-addressing table of 2^bits slots, at most a
+// quarter full up to 512 members and half full beyond.  An id's home is the
+// top bits of its multiplicative hash (a trimmed core's members are runs of
+// consecutive ids, which an identity hash would chain together); a slot holds
+// 20 other hash bits and the member's list position.  The induced rows look
+// every out-neighbour of every member up: a probe or two replaces a binary
+// search of the list (~9 dependent shared-memory reads at 500 members).
+__host__ __device__ __forceinline__ int tab_bits(uint32_t d) {
+  int b = 6;
+  while ((1u << b) < 4 * d && ((1u << b) < 2048 || (1u << b) < 2 * d)) ++b;
+  return b;
+}
+constexpr uint32_t kTabEmpty = 0xffffffffu;  // no entry: positions stay below 4095
+__device__ __forceinline__ void tab_insert(uint32_t *tab, int bits, uint32_t y, int pos) {
+  const uint32_t h = y * 0x9E3779B1u, mask = (1u << bits) - 1u, e = (h << 12) | (uint32_t)pos;
+  uint32_t at = h >> (32 - bits);
+  while (atomicCAS(tab + at, kTabEmpty, e) != kTabEmpty) at = (at + 1) & mask;
+}
+// Position of y in list, or -1.
+__device__ __forceinline__ int tab_find(const uint32_t *tab, int bits, const uint32_t *list, uint32_t y) {
+  const uint32_t h = y * 0x9E3779B1u, mask = (1u << bits) - 1u;
+  for (uint32_t at = h >> (32 - bits);; at = (at + 1) & mask) {
+    const uint32_t e = tab[at];
+    if (e == kTabEmpty) return -1;
+    if (((e >> 12) ^ h) << 12 == 0 && list[e & 4095u] == y) return (int)(e & 4095u);
+  }
+}
+
+// A vertex's bitmap row, if it has one: the word its out-neighbours' bits start
+// at in a.bits, the id of the first bit and the number of ids it covers.
+constexpr uint32_t kNoBitRow = 0xffffffffu;
+__device__ __forceinline__ uint4 bit_row(const PassArgs &a, uint32_t x) {
+  return a.bit_rows ? __ldg(a.bit_rows + x) : make_uint4(kNoBitRow, 0u, 0u, 0u);
+}
+// Bit of id y in the row starting at word `row`, id `first`, `span` ids long.
+__device__ __forceinline__ bool bit_at(const PassArgs &a, uint32_t row, uint32_t first, uint32_t span, uint32_t y) {
+  const uint32_t t = y - first;
+  return t < span && ((__ldg(a.bits + row + (t >> 5)) >> (t & 31)) & 1u);
+}
+
+// Shared-memory add of a 64-bit word by its native 32-bit halves (the 64-bit
+// form is a compare-and-swap loop, which serialises when warps meet in a word).
+__device__ __forceinline__ void shared_add(unsigned long long *p, unsigned long long x) {
+  uint32_t *w = reinterpret_cast<uint32_t *>(p);
+  const uint32_t lo = (uint32_t)x;
+  const uint32_t hi = (uint32_t)(x >> 32) + (atomicAdd(w, lo) + lo < lo);
+  if (hi) atomicAdd(w + 1, hi);
+}
 template <int MODE>
 struct SmemS {
   uint32_t list[kSMaxD];
+  uint32_t tab[4 * kSMaxD];
   unsigned long long rows[kSMaxD];
   unsigned long long base[kSMaxD + 1];  // SEQ: pass-start r; ORDER: keys
   unsigned long long acc[kSMaxD + 1];   // SEQ: per-root increments
@@ -202,39 +251,83 @@ __global__ void __launch_bounds__(kWarpsS * 32) tier_s_kernel(PassArgs a) {
     for (int i = lane; i < kSMaxD; i += 32) sm.rows[i] = 0;
     __syncwarp();
     if (K >= 3) {
-      // Row i: out-neighbours of list[i] inside N+(s), by merging the two
-      // ascending lists (MakeSubgraph's induced adjacency, :104-113).
-      for (int i = lane; i < d; i += 32) {
-        const uint32_t x = sm.list[i];
-        const uint64_t xe = a.off[x + 1];
-        unsigned long long row = 0;
-        int j = 0;
-        for (uint64_t e = a.off[x]; e < xe && j < i; ++e) {
-          const uint32_t y = a.cols[e];
-          while (j < i && sm.list[j] < y) ++j;
-          if (j < i && sm.list[j] == y) row |= 1ull << j;
-        }
-        if constexpr (MODE == MODE_SEQ) {
+      // Row i: out-neighbours of list[i] inside N+(s) (MakeSubgraph's induced
+      // adjacency, :104-113).  A member with a bitmap row is asked about every
+      // member before it at once, a lane each; the others' out-lists are
+      // walked, a lane per row.
+      const uint32_t y0 = lane < d ? sm.list[lane] : 0u, y1 = lane + 32 < d ? sm.list[lane + 32] : 0u;
+      const uint4 b0 = lane < d ? bit_row(a, y0) : make_uint4(0, 0, 0, 0);
+      const uint4 b1 = lane + 32 < d ? bit_row(a, y1) : make_uint4(0, 0, 0, 0);
+#pragma unroll 4
+      for (int i = 1; i < d; ++i) {
+        const uint32_t bo = __shfl_sync(KCL_FULL, i < 32 ? b0.x : b1.x, i & 31);
+        const uint32_t bf = __shfl_sync(KCL_FULL, i < 32 ? b0.y : b1.y, i & 31);
+        const uint32_t bs = __shfl_sync(KCL_FULL, i < 32 ? b0.z : b1.z, i & 31);  // 0: no row, no hit
+        const bool h0 = lane < i && bit_at(a, bo, bf, bs, y0);
+        const bool h1 = lane + 32 < i && bit_at(a, bo, bf, bs, y1);
+        const uint32_t m0 = __ballot_sync(KCL_FULL, h0);
+        const uint32_t m1 = i > 32 ? __ballot_sync(KCL_FULL, h1) : 0u;
+        if (lane == 0) sm.rows[i] = (unsigned long long)m1 << 32 | m0;
+      }
+      const bool w0 = lane < d && b0.x == kNoBitRow, w1 = lane + 32 < d && b1.x == kNoBitRow;
+      if (__any_sync(KCL_FULL, w0 || w1)) {
+        const int tb = tab_bits((uint32_t)d);
+        for (int i = lane; i < 1 << tb; i += 32) sm.tab[i] = kTabEmpty;
+        __syncwarp();
+        for (int i = lane; i < d; i += 32) tab_insert(sm.tab, tb, sm.list[i], i);
+        __syncwarp();
+        for (int i = lane; i < d; i += 32) {
+          if (!(i < 32 ? w0 : w1) || i == 0) continue;
+          const uint32_t x = sm.list[i], top = sm.list[i - 1];
+          const uint64_t xe = a.off[x + 1];
+          unsigned long long row = 0;
+          for (uint64_t e = a.off[x]; e < xe; e += 4) {
+            uint32_t y[4];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) y[b] = e + b < xe ? a.cols[e + b] : 0xffffffffu;
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+              if (y[b] <= top) {
+                const int j = tab_find(sm.tab, tb, sm.list, y[b]);
+                if (j >= 0) row |= 1ull << j;
+              }
+            if (y[3] > top) break;  // ascending: no later neighbour is in list[0, i)
+          }
           sm.rows[i] = row;
-        } else if constexpr (MODE == MODE_COUNT) {
-          atomicOr(&sm.rows[i], row);
-          unsigned long long it = row;
-          while (it) {
-            const int j2 = __ffsll((long long)it) - 1;
-            it &= it - 1;
-            atomicOr(&sm.rows[j2], 1ull << i);
-          }
-        } else {
-          const int ri = sm.rank[i];
-          unsigned long long it = row;
-          while (it) {
-            const int j2 = __ffsll((long long)it) - 1;
-            it &= it - 1;
-            const int rj = sm.rank[j2];
-            const int lo = ri < rj ? ri : rj, hi = ri < rj ? rj : ri;
-            atomicOr(&sm.rows[lo], 1ull << hi);
-          }
         }
+      }
+      __syncwarp();
+      if constexpr (MODE != MODE_SEQ) {
+        // COUNT: symmetric rows; ORDER: rows by key rank, upward.  A lane reads
+        // its whole row off the lower triangle: no bit is set by an atomic
+        // (lanes meeting in a word made the former scatter the kernel's
+        // longest phase, 228 us of a 64-member root's 245).
+        const uint32_t *half = reinterpret_cast<const uint32_t *>(sm.rows);
+        unsigned long long full[2] = {0, 0};
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int p = lane + 32 * q;
+          if (32 * q >= d) break;
+          const int i = MODE == MODE_ORDER ? (p < d ? sm.inv[p] : 0) : p;
+          uint32_t w[2] = {0, 0};
+#pragma unroll
+          for (int z = 0; z < 2; ++z) {
+            if (MODE == MODE_ORDER && z < q) continue;  // upward: higher ranks only
+            const int end = d - 32 * z < 32 ? d - 32 * z : 32;
+            for (int b = 0; b < end; ++b) {
+              const int j = MODE == MODE_ORDER ? sm.inv[32 * z + b] : 32 * z + b;
+              const int hi = MODE == MODE_ORDER && i > j ? i : j, lo = MODE == MODE_ORDER && i > j ? j : i;
+              if ((half[2 * hi + (lo >> 5)] >> (lo & 31)) & 1u) w[z] |= 1u << b;  // rows hold bits below their own
+            }
+          }
+          full[q] = (unsigned long long)w[1] << 32 | w[0];
+          if constexpr (MODE == MODE_ORDER) full[q] &= ~((2ull << p) - 1ull);
+          else full[q] |= p < d ? sm.rows[p] : 0ull;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+          if (lane + 32 * q < d) sm.rows[lane + 32 * q] = full[q];
       }
       __syncwarp();
     }
@@ -250,7 +343,7 @@ __global__ void __launch_bounds__(kWarpsS * 32) tier_s_kernel(PassArgs a) {
         auto close = [&](int i) {
           if (!dl[i]) return;
           if (a.shared_loads) atomicAdd(a.out + (i < d ? sm.list[i] : s), (unsigned long long)dl[i]);
-          else atomicAdd(&sm.acc[i], (unsigned long long)dl[i]);
+          else shared_add(&sm.acc[i], dl[i]);
           dl[i] = 0;
         };
         unsigned long long it = C;
@@ -503,7 +596,7 @@ __host__ __device__ inline size_t seq_warp_words(int k, uint32_t dmax, bool rows
 // Shared-memory layout of a tier M / L CTA (dmax = largest out-degree the
 // launch allows, NW warps).  Tier L keeps `rows` in a global slab instead.
 struct LayoutM {
-  size_t list, rows, base, acc, rel, rank, inv, dl, cbuf, total;
+  size_t list, tab, rows, base, acc, rel, rank, inv, dl, cbuf, total;
 };
 // Per-warp scratch of the k = 4 counting path (edges_in): P's words and its
 // members, compacted.
@@ -514,6 +607,7 @@ __host__ __device__ inline LayoutM layout_m(int mode, int k, uint32_t dmax, int 
   const size_t W = (dmax + 31) / 32;
   size_t at = 0;
   L.list = at; at = align16(at + (size_t)dmax * 4);
+  L.tab = at; at = align16(at + ((size_t)4 << tab_bits(dmax)));
   L.rows = at;
   if (rows_in_smem) at = align16(at + (mode == MODE_SEQ ? (size_t)tri_off(dmax) : (size_t)dmax * W) * 4);
   L.base = at; if (mode != MODE_COUNT) at = align16(at + (size_t)(dmax + 1) * 8);
@@ -921,7 +1015,7 @@ struct TinyStream {
       const int i = 32 * q + lane;
       if (i < nc) {
         const uint32_t id = list[i], d = v[q] - rel[id];
-        if (d) atomicAdd(acc + id, (unsigned long long)d);
+        if (d) shared_add(acc + id, d);
       }
     }
     return c;
@@ -979,7 +1073,7 @@ struct PairLevel {
 
   __device__ __forceinline__ void put(uint32_t id, uint32_t v0, uint32_t v) const {
     if constexpr (ACC) {
-      if (v != v0) atomicAdd(acc + id, (unsigned long long)(v - v0));
+      if (v != v0) shared_add(acc + id, v - v0);
     } else {
       val[id] = v;
     }
@@ -1519,13 +1613,13 @@ __device__ __forceinline__ void seq_streams(uint32_t *next, int d, const uint32_
             ts.lane = lane;
             c1 = ts.template run<K>(rows, list, (int)nc, rel, acc, c0);
           }
-          if (lane == 0 && c1 != c0) atomicAdd(&acc[g0], (unsigned long long)(c1 - c0));
+          if (lane == 0 && c1 != c0) shared_add(&acc[g0], c1 - c0);
           continue;
         }
         if constexpr (K == 4) {
           uint32_t c = c0;
           if (PairLevel<true>{rows, const_cast<uint32_t *>(rel), acc, pair, lane}(C.w[0], c)) {
-            if (lane == 0 && c != c0) atomicAdd(&acc[g0], (unsigned long long)(c - c0));
+            if (lane == 0 && c != c0) shared_add(&acc[g0], c - c0);
             continue;
           }
         } else {
@@ -1535,9 +1629,9 @@ __device__ __forceinline__ void seq_streams(uint32_t *next, int d, const uint32_
           __syncwarp();
           for_members<1>(C, lane, [&](int i) {
             const uint32_t delta = cur[i] - rel[i];
-            if (delta) atomicAdd(&acc[i], (unsigned long long)delta);
+            if (delta) shared_add(&acc[i], delta);
           });
-          if (lane == 0 && c1 != c0) atomicAdd(&acc[g0], (unsigned long long)(c1 - c0));
+          if (lane == 0 && c1 != c0) shared_add(&acc[g0], c1 - c0);
           continue;
         }
       }
@@ -1587,9 +1681,9 @@ __device__ __forceinline__ void seq_streams(uint32_t *next, int d, const uint32_
       for_members<WPL>(C, lane, [&](int i) {
         const unsigned long long rel = base[i] - off;
         const uint32_t delta = cur[i] - (uint32_t)(rel < cap ? rel : cap);
-        if (delta) atomicAdd(&acc[i], (unsigned long long)delta);
+        if (delta) shared_add(&acc[i], delta);
       });
-      if (lane == 0 && c1 != c0) atomicAdd(&acc[g0], (unsigned long long)(c1 - c0));
+      if (lane == 0 && c1 != c0) shared_add(&acc[g0], c1 - c0);
     } else {
       for_members<WPL>(C, lane, [&](int i) { cur[i] = 0; });
       const Vals64<(K >= 6)> va{base, cur};
@@ -1597,9 +1691,9 @@ __device__ __forceinline__ void seq_streams(uint32_t *next, int d, const uint32_
       const unsigned long long c1 = seq_rec<K - 2, WPL, Vals64<(K >= 6)>, false>(C, c0, rows, va, 0u, lane, err);
       for_members<WPL>(C, lane, [&](int i) {
         const uint32_t delta = cur[i];
-        if (delta) atomicAdd(&acc[i], (unsigned long long)delta);
+        if (delta) shared_add(&acc[i], delta);
       });
-      if (lane == 0 && c1 != c0) atomicAdd(&acc[g0], c1 - c0);
+      if (lane == 0 && c1 != c0) shared_add(&acc[g0], c1 - c0);
     }
   }
 }
@@ -1725,6 +1819,7 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
   const int dmax = (int)a.dmax;
   const LayoutM lay = layout_m(MODE, K, a.dmax, NW, ROWS_IN_SMEM);
   uint32_t *list = reinterpret_cast<uint32_t *>(smem_raw + lay.list);
+  uint32_t *tab = reinterpret_cast<uint32_t *>(smem_raw + lay.tab);
   uint32_t *rows = ROWS_IN_SMEM ? reinterpret_cast<uint32_t *>(smem_raw + lay.rows)
                                 : a.slab + (size_t)blockIdx.x * a.slab_words;
   unsigned long long *base = reinterpret_cast<unsigned long long *>(smem_raw + lay.base);
@@ -1745,6 +1840,14 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
     for (int i = tid; i <= dmax; i += NW * 32) acc[i] = 0;
     for (int i = lane; i <= dmax; i += 32) dl[i] = 0;
   }
+  __shared__ unsigned long long s_min[MODE == MODE_SEQ ? 32 : 1];
+  // The CTA's smallest x (a warp's share each; one barrier).
+  auto cta_min = [&](unsigned long long x) {
+    x = warp_min_u64(x);
+    if (lane == 0) s_min[wid] = x;
+    __syncthreads();
+    return warp_min_u64(lane < NW ? s_min[lane] : ~0ull);
+  };
   bool stealing = false;  // warp 0's view (uniform across its lanes)
   __syncthreads();
   for (;;) {
@@ -1760,7 +1863,6 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
         s_idx = idx;
         s_tau = 0;
         s_sum = 0;
-        s_off = ~0ull;
         if (a.active && idx != UINT32_MAX) a.active[blockIdx.x] = idx;  // visible to thieves
       }
     }
@@ -1798,6 +1900,8 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
     const int row_words = MODE == MODE_SEQ ? (int)tri_off((uint32_t)d) : d * W;
     for (int i = tid; i < d; i += NW * 32) list[i] = lcols[o + i];
     for (int i = tid; i < row_words; i += NW * 32) rows[i] = 0;
+    const int tb = tab_bits((uint32_t)d);
+    for (int i = tid; i < 1 << tb; i += NW * 32) tab[i] = kTabEmpty;
     if constexpr (MODE == MODE_ORDER) {
       for (int i = tid; i < d; i += NW * 32) base[i] = vertex_key(a, a.cols[o + i]);
       if (tid == 0) base[d] = vertex_key(a, s);
@@ -1813,10 +1917,8 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
           base[i] = __ldcg(a.out + (i < d ? a.cols[o + i] : s));
           mn = base[i] < mn ? base[i] : mn;
         }
-        mn = warp_min_u64(mn);
-        if (lane == 0) atomicMin(&s_off, mn);
-        __syncthreads();
-        const unsigned long long off = s_off;
+        const unsigned long long off = cta_min(mn);
+        if (tid == 0) s_off = off;
         for (int i = tid; i <= d; i += NW * 32) {
           const unsigned long long v = base[i] - off;
           cur[i] = v < kSharedCap ? (uint32_t)v : kSharedCap;
@@ -1829,10 +1931,7 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
           mn = v < mn ? v : mn;
         }
         if constexpr (K >= 4 && ROWS_IN_SMEM) {
-          mn = warp_min_u64(mn);
-          if (lane == 0) atomicMin(&s_off, mn);
-          __syncthreads();
-          const unsigned long long off = s_off;
+          const unsigned long long off = cta_min(mn);
           for (int i = tid; i <= d; i += NW * 32) {
             const unsigned long long v = base[i] - off;
             rel[i] = v < kRelCap ? (uint32_t)v : kRelCap;
@@ -1860,28 +1959,67 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
       __syncthreads();
     }
     if (K >= 3) {
+      for (int i = tid; i < d; i += NW * 32) tab_insert(tab, tb, list[i], i);
+      __syncthreads();
       // Row i: N+(list[i]) ∩ N+(s) (MakeSubgraph's induced adjacency,
-      // kCDensestNoAtom.c:104-113), one warp per row, a lane per out-neighbour.
-      for (int i = wid; i < d; i += NW) {
-        if (i == 0) continue;
-        const uint32_t x = list[i];
-        const uint32_t top = list[i - 1];
-        const uint64_t xe = a.off[x + 1];
-        for (uint64_t e = a.off[x] + lane; e < xe; e += 32) {
-          const uint32_t y = a.cols[e];
-          if (y > top) break;  // ascending: no later neighbour is in list[0, i)
-          const int j = lower_bound_u32(list, i, y);
-          if (list[j] != y) continue;
-          if constexpr (MODE == MODE_SEQ) {
-            atomicOr(&rows[(size_t)tri_off((uint32_t)i) + (j >> 5)], 1u << (j & 31));
-          } else if constexpr (MODE == MODE_COUNT) {
-            atomicOr(&rows[(size_t)i * W + (j >> 5)], 1u << (j & 31));
-            atomicOr(&rows[(size_t)j * W + (i >> 5)], 1u << (i & 31));
-          } else {
-            const int ri = rank[i], rj = rank[j];
-            const int lo = ri < rj ? ri : rj, hi = ri < rj ? rj : ri;
-            atomicOr(&rows[(size_t)lo * W + (hi >> 5)], 1u << (hi & 31));
+      // kCDensestNoAtom.c:104-113), one warp per row.  A member with a bitmap
+      // row is asked about 32 earlier members at a time (a word of row i per
+      // ballot); the others' out-lists are walked, a lane per out-neighbour,
+      // and looked up in the table.  Latency bounds this phase (a row's
+      // offsets, its list and the look-ups are dependent reads), and it was 42
+      // to 68 % of a CTA's time once the streams were cheap: walking every
+      // list with a binary search, the k = 3 wave passes of an RMAT-17 graph
+      // took 6.0 ms, now 3.2; the k = 4 count of RMAT-18 4.1 -> 2.2 ms, a Seq
+      // pass over the RMAT-18 core 1.36 -> 1.03 ms.
+      auto put = [&](int i, int j) {  // j, before i, is its neighbour
+        if constexpr (MODE == MODE_SEQ) {
+          atomicOr(&rows[(size_t)tri_off((uint32_t)i) + (j >> 5)], 1u << (j & 31));
+        } else if constexpr (MODE == MODE_COUNT) {
+          atomicOr(&rows[(size_t)i * W + (j >> 5)], 1u << (j & 31));
+          atomicOr(&rows[(size_t)j * W + (i >> 5)], 1u << (i & 31));
+        } else {
+          const int ri = rank[i], rj = rank[j];
+          const int lo = ri < rj ? ri : rj, hi = ri < rj ? rj : ri;
+          atomicOr(&rows[(size_t)lo * W + (hi >> 5)], 1u << (hi & 31));
+        }
+      };
+      for (int r0 = wid; r0 < d; r0 += NW * 32) {
+        // this warp's next 32 rows: r0, r0 + NW, ...
+        const int ri = r0 + NW * lane;
+        const uint4 br = ri < d ? bit_row(a, list[ri]) : make_uint4(kNoBitRow, 0u, 0u, 0u);
+        for (int q = 0, i = r0; q < 32 && i < d; ++q, i += NW) {
+          const uint32_t bo = __shfl_sync(KCL_FULL, br.x, q), bf = __shfl_sync(KCL_FULL, br.y, q);
+          const uint32_t bs = __shfl_sync(KCL_FULL, br.z, q);
+          if (i == 0) continue;
+          if (bo != kNoBitRow) {
+            const int nw = (i + 31) >> 5;
+#pragma unroll 4
+            for (int w = 0; w < nw; ++w) {
+              const int j = (w << 5) | lane;
+              const bool hit = j < i && bit_at(a, bo, bf, bs, list[j]);
+              if constexpr (MODE == MODE_SEQ) {
+                const uint32_t m = __ballot_sync(KCL_FULL, hit);
+                if (lane == 0) rows[(size_t)tri_off((uint32_t)i) + w] = m;
+              } else if constexpr (MODE == MODE_COUNT) {
+                const uint32_t m = __ballot_sync(KCL_FULL, hit);
+                if (lane == 0 && m) atomicOr(&rows[(size_t)i * W + w], m);
+                if (hit) atomicOr(&rows[(size_t)j * W + (i >> 5)], 1u << (i & 31));
+              } else if (hit) {
+                put(i, j);
+              }
+            }
+            continue;
           }
+          const uint32_t x = list[i];
+          const uint32_t top = list[i - 1];
+          const uint64_t xe = a.off[x + 1];
+          for (uint64_t e = a.off[x] + lane; e < xe; e += 32) {
+            const uint32_t y = a.cols[e];
+            if (y > top) break;  // ascending: no later neighbour is in list[0, i)
+            const int j = tab_find(tab, tb, list, y);
+            if (j >= 0) put(i, j);
+          }
+          __syncwarp();
         }
       }
       __syncthreads();
@@ -1942,7 +2080,7 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
           }
         }
       }
-      if (lane == 0 && mine) atomicAdd(&s_sum, mine);
+      if (lane == 0 && mine) shared_add(&s_sum, mine);
       __syncthreads();
       if (tid == 0 && s_sum && !(MODE == MODE_COUNT && a.list_off)) {
         atomicAdd(&a.out[s], s_sum);

@@ -160,6 +160,8 @@ kclpp_status peel_recount_run(PeelRecount *P, uint32_t nroots, const uint64_t *l
   dev::PassArgs a{};
   a.off = graph_dev_offsets(P->g);
   a.cols = graph_dev_cols(P->g);
+  a.bit_rows = graph_dev_bit_rows(P->g);
+  a.bits = graph_dev_bits(P->g);
   a.err = ctx_err_word(c);
   a.list_off = P->d_loff;
   a.list_cols = P->d_lcols;
