@@ -15,6 +15,7 @@
 #include <numeric>
 
 #include "kclpp_dev.cuh"
+#include "kclpp_extract.cuh"
 #include "kclpp_internal.h"
 
 namespace kclpp {
@@ -115,6 +116,10 @@ struct kclpp_graph {
   uint32_t *d_slab = nullptr;
   uint64_t slab_words = 0;
   int slab_ctas = 0;
+  // reports: the order's scratch, the order itself and the best prefix
+  OrderScratch ord;
+  uint32_t *d_order = nullptr;
+  PrefixBest *d_best = nullptr;
 };
 
 // ---------------------------------------------------------------------------
@@ -138,7 +143,8 @@ __global__ void k_scatter_level(unsigned long long *tent, const unsigned long lo
 }
 
 __global__ void k_count_edges(const uint32_t *src, const uint32_t *cols, uint64_t m, const uint32_t *level,
-                              uint32_t nstar, unsigned long long *out) {
+                              const uint32_t *prefix, unsigned long long *out) {
+  const uint32_t nstar = prefix ? *prefix : 1u;
   unsigned long long c = 0;
   for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x)
     c += (level[src[e]] < nstar && level[cols[e]] < nstar);
@@ -393,6 +399,8 @@ static kclpp_status upload_graph(kclpp_ctx *c, kclpp_graph *g) {
 
 static void free_graph_dev(kclpp_graph *g) {
   cudaFree(g->d_bit_rows); cudaFree(g->d_bits);
+  order_scratch_free(g->ord);
+  cudaFree(g->d_order); cudaFree(g->d_best);
   cudaFree(g->d_off); cudaFree(g->d_cols); cudaFree(g->d_src); cudaFree(g->d_roots);
   cudaFree(g->d_a); cudaFree(g->d_b); cudaFree(g->d_rho); cudaFree(g->d_level);
   cudaFree(g->d_work); cudaFree(g->d_task); cudaFree(g->d_scalar); cudaFree(g->d_slab);
@@ -1434,7 +1442,7 @@ kclpp_status kclpp_count_edges(kclpp_ctx *c, const kclpp_graph *gc, uint32_t num
   const uint64_t m = g->dag.m();
   if (m) {
     k_count_edges<<<std::min(blocks_for(m), c->num_sms * 8), 256, 0, c->stream>>>(g->d_src, g->d_cols, m,
-                                                                               g->d_level, 1u, g->d_scalar);
+                                                                               g->d_level, nullptr, g->d_scalar);
     KCL_CUDA(cudaGetLastError());
     c->launches++;
   }
@@ -1446,30 +1454,50 @@ kclpp_status kclpp_count_edges(kclpp_ctx *c, const kclpp_graph *gc, uint32_t num
 }
 
 // Shared tail of both extractions: PAVA pass on the device, CountEdges.
-static kclpp_status pava_and_edges(kclpp_ctx *c, kclpp_graph *g, int k, const std::vector<uint32_t> &level,
-                                   std::vector<uint64_t> &tent) {
-  const uint32_t n = g->dag.n;
-  KCL_CUDA(cudaMemcpyAsync(g->d_level, level.data(), (size_t)n * 4, cudaMemcpyHostToDevice, c->stream));
-  KCL_TRY(pava_dev(c, g, k, g->d_level, g->d_b));
-  tent.resize(n);
-  KCL_CUDA(cudaMemcpyAsync(tent.data(), g->d_b, (size_t)n * 8, cudaMemcpyDeviceToHost, c->stream));
-  return check_err(c);
+// The device part of a report (kCDensestNoAtom.c:330-349): the vertices by
+// decreasing key into d_order / d_level, the prefix clique counts (PAVA) into
+// d_b, the first strictly densest prefix and the edges inside it.  keys is a
+// host vector.  The order's head, which the bound scan reads, is left in head.
+struct Report {
+  PrefixBest best;
+  std::vector<uint32_t> head;  // the first vertices of the order
+};
+constexpr uint32_t kReportHead = 4096;
+
+static kclpp_status order_head(kclpp_ctx *c, kclpp_graph *g, uint32_t upto, Report *r) {
+  const uint32_t have = (uint32_t)r->head.size();
+  if (upto <= have) return KCLPP_OK;
+  r->head.resize(upto);
+  KCL_CUDA(cudaMemcpyAsync(r->head.data() + have, g->d_order + have, (size_t)(upto - have) * 4,
+                           cudaMemcpyDeviceToHost, c->stream));
+  KCL_CUDA(cudaStreamSynchronize(c->stream));
+  return KCLPP_OK;
 }
 
-static kclpp_status edges_in_prefix(kclpp_ctx *c, kclpp_graph *g, uint32_t nstar, uint32_t *m_out) {
-  KCL_CUDA(cudaMemsetAsync(g->d_scalar, 0, 8, c->stream));
+static kclpp_status report_dev(kclpp_ctx *c, kclpp_graph *g, int k, const uint64_t *keys, Report *r) {
+  const uint32_t n = g->dag.n;
+  cudaError_t e = order_scratch_make(g->ord, n);
+  if (e != cudaSuccess) return set_error(KCLPP_ERR_NOMEM, "report: %s", cudaGetErrorString(e));
+  KCL_TRY(dalloc(&g->d_order, n));
+  KCL_TRY(dalloc(&g->d_best, 1));
+  uint64_t top = 0;
+  for (uint32_t i = 0; i < n; ++i) top |= keys[i];
+  KCL_CUDA(cudaMemcpyAsync(g->d_a, keys, (size_t)n * 8, cudaMemcpyHostToDevice, c->stream));
+  KCL_CUDA(order_by_key(g->d_a, n, top, g->ord, g->d_order, g->d_level, c->stream, &c->launches));
+  KCL_TRY(pava_dev(c, g, k, g->d_level, g->d_b));
+  KCL_CUDA(densest_prefix(g->d_b, n, g->ord, g->d_best, c->stream, &c->launches));
   const uint64_t m = g->dag.m();
   if (m) {
-    k_count_edges<<<std::min(blocks_for(m), c->num_sms * 8), 256, 0, c->stream>>>(g->d_src, g->d_cols, m,
-                                                                               g->d_level, nstar, g->d_scalar);
+    k_count_edges<<<std::min(blocks_for(m), c->num_sms * 8), 256, 0, c->stream>>>(g->d_src, g->d_cols, m, g->d_level,
+                                                                               &g->d_best->n, &g->d_best->edges);
     KCL_CUDA(cudaGetLastError());
     c->launches++;
   }
-  unsigned long long h = 0;
-  KCL_CUDA(cudaMemcpyAsync(&h, g->d_scalar, 8, cudaMemcpyDeviceToHost, c->stream));
-  KCL_TRY(check_err(c));
-  *m_out = (uint32_t)h;
-  return KCLPP_OK;
+  const uint32_t head = std::min(n, kReportHead);
+  r->head.resize(head);
+  KCL_CUDA(cudaMemcpyAsync(&r->best, g->d_best, sizeof r->best, cudaMemcpyDeviceToHost, c->stream));
+  KCL_CUDA(cudaMemcpyAsync(r->head.data(), g->d_order, (size_t)head * 4, cudaMemcpyDeviceToHost, c->stream));
+  return check_err(c);
 }
 
 extern "C++" {
@@ -1493,22 +1521,6 @@ static double upper_bound_scan(uint32_t n, int k, NextLoad next_load) {
   }
   return ub;
 }
-
-// kCDensestNoAtom.c:342-349: the first strictly largest prefix density of the
-// exact prefix clique counts (integer accumulator).
-static void densest_prefix_u64(const std::vector<uint64_t> &tent, kclpp_densest_info *info) {
-  double density = -1;
-  unsigned long long sum = 0;
-  for (uint32_t i = 0; i < (uint32_t)tent.size(); ++i) {
-    sum += tent[i];
-    if ((double)sum / (i + 1) > density) {
-      density = (double)sum / (i + 1);
-      info->n = i + 1;
-      info->cliques = sum;
-    }
-  }
-  info->density = density;
-}
 }  // extern "C++"
 
 kclpp_status kclpp_extract_densest_seq(kclpp_ctx *c, const kclpp_graph *gc, int k, uint32_t T, const uint64_t *r,
@@ -1522,18 +1534,22 @@ kclpp_status kclpp_extract_densest_seq(kclpp_ctx *c, const kclpp_graph *gc, int 
   memset(info, 0, sizeof *info);
   const uint32_t n = g->dag.n;
   if (!n) return KCLPP_OK;
-  std::vector<uint32_t> reordered(n), level(n);
-  KCL_TRY(kclpp_sort_by_r_u64(c, n, r, reordered.data(), level.data()));
-  std::vector<uint64_t> tent;
-  KCL_TRY(pava_and_edges(c, g, k, level, tent));
-  densest_prefix_u64(tent, info);
-  KCL_TRY(edges_in_prefix(c, g, info->n, &info->m));
+  Report rp;
+  KCL_TRY(report_dev(c, g, k, r, &rp));
+  info->n = rp.best.n;
+  info->cliques = rp.best.cliques;
+  info->density = rp.best.density;
+  info->m = (uint32_t)rp.best.edges;
+  if (reordered_out) KCL_TRY(order_head(c, g, n, &rp));
   unsigned long long sum = 0;
+  kclpp_status more = KCLPP_OK;
   info->ub = upper_bound_scan(n, k, [&](uint32_t i) {
-    sum += r[reordered[i]];
+    if (i == rp.head.size() && (more = order_head(c, g, n, &rp)) != KCLPP_OK) return -1.0;  // ends the scan
+    sum += r[rp.head[i]];
     return (double)sum / T;
   });
-  if (reordered_out) memcpy(reordered_out, reordered.data(), (size_t)n * 4);
+  KCL_TRY(more);
+  if (reordered_out) memcpy(reordered_out, rp.head.data(), (size_t)n * 4);
   return KCLPP_OK;
 }
 
@@ -1547,30 +1563,50 @@ kclpp_status kclpp_extract_densest_sim(kclpp_ctx *c, const kclpp_graph *gc, int 
   memset(info, 0, sizeof *info);
   const uint32_t n = g->dag.n;
   if (!n) return KCLPP_OK;
-  std::vector<uint32_t> reordered(n), level(n);
-  KCL_TRY(kclpp_sort_by_r_f64(c, n, rho, reordered.data(), level.data()));
-  std::vector<uint64_t> tent;
-  KCL_TRY(pava_and_edges(c, g, k, level, tent));
-  // kCDensestCmpSync.c:354-361 (double accumulator)
-  double density = -1, sum = 0;
-  uint64_t isum = 0;
-  for (uint32_t i = 0; i < n; ++i) {
-    sum += (double)tent[i];
-    isum += tent[i];
-    if (sum / (i + 1) > density) {
-      density = sum / (i + 1);
-      info->n = i + 1;
-      info->cliques = isum;
+  std::vector<uint64_t> keys(n);
+  for (uint32_t i = 0; i < n; ++i) keys[i] = (unsigned long long)rho[i];
+  Report rp;
+  KCL_TRY(report_dev(c, g, k, keys.data(), &rp));
+  info->n = rp.best.n;
+  info->cliques = rp.best.cliques;
+  info->density = rp.best.density;
+  info->m = (uint32_t)rp.best.edges;
+  if (rp.best.total > (1ull << 53)) {
+    // kCDensestCmpSync.c:354-361 sums in a double: beyond 2^53 its roundings
+    // are its own, so the scan runs as written there.
+    std::vector<uint64_t> tent(n);
+    std::vector<uint32_t> level(n);
+    KCL_CUDA(cudaMemcpyAsync(tent.data(), g->d_b, (size_t)n * 8, cudaMemcpyDeviceToHost, c->stream));
+    KCL_CUDA(cudaMemcpyAsync(level.data(), g->d_level, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream));
+    KCL_CUDA(cudaStreamSynchronize(c->stream));
+    double density = -1, dsum = 0;
+    uint64_t isum = 0;
+    for (uint32_t i = 0; i < n; ++i) {
+      dsum += (double)tent[i];
+      isum += tent[i];
+      if (dsum / (i + 1) > density) {
+        density = dsum / (i + 1);
+        info->n = i + 1;
+        info->cliques = isum;
+      }
     }
+    info->density = density;
+    uint64_t inside = 0;
+    for (uint32_t s = 0; s < n; ++s)
+      if (level[s] < info->n)
+        for (uint64_t e = g->dag.off[s]; e < g->dag.off[s + 1]; ++e) inside += level[g->dag.cols[e]] < info->n;
+    info->m = (uint32_t)inside;
   }
-  info->density = density;
-  KCL_TRY(edges_in_prefix(c, g, info->n, &info->m));
-  sum = 0;
+  if (reordered_out) KCL_TRY(order_head(c, g, n, &rp));
+  double sum = 0;
+  kclpp_status more = KCLPP_OK;
   info->ub = upper_bound_scan(n, k, [&](uint32_t i) {
-    sum += rho[reordered[i]];
+    if (i == rp.head.size() && (more = order_head(c, g, n, &rp)) != KCLPP_OK) return -1.0;  // ends the scan
+    sum += rho[rp.head[i]];
     return sum;
   });
-  if (reordered_out) memcpy(reordered_out, reordered.data(), (size_t)n * 4);
+  KCL_TRY(more);
+  if (reordered_out) memcpy(reordered_out, rp.head.data(), (size_t)n * 4);
   return KCLPP_OK;
 }
 
@@ -1647,6 +1683,7 @@ kclpp_status ctx_check_err(kclpp_ctx *c) { return check_err(c); }
 const HostDag &graph_dag(const kclpp_graph *g) { return g->dag; }
 const uint64_t *graph_dev_offsets(const kclpp_graph *g) { return g->d_off; }
 const uint32_t *graph_dev_cols(const kclpp_graph *g) { return g->d_cols; }
+const uint32_t *graph_dev_count_roots(const kclpp_graph *g) { return g->d_roots + g->sched_base[0]; }
 const uint4 *graph_dev_bit_rows(const kclpp_graph *g) { return g->d_bit_rows; }
 const uint32_t *graph_dev_bits(const kclpp_graph *g) { return g->d_bits; }
 int graph_device(const kclpp_graph *g) { return g->device; }
@@ -1758,12 +1795,12 @@ kclpp_status kclpp_extract_densest_seq_warm(kclpp_ctx *c, const kclpp_graph *gc,
   if (!n) return KCLPP_OK;
   // Densest prefix in the order of r (warm start included): the same scan as
   // kCDensestNoAtom.c:341-349 on exact prefix clique counts.
-  std::vector<uint32_t> reordered(n), level(n);
-  KCL_TRY(kclpp_sort_by_r_u64(c, n, r, reordered.data(), level.data()));
-  std::vector<uint64_t> tent;
-  KCL_TRY(pava_and_edges(c, g, k, level, tent));
-  densest_prefix_u64(tent, info);
-  KCL_TRY(edges_in_prefix(c, g, info->n, &info->m));
+  Report rp;
+  KCL_TRY(report_dev(c, g, k, r, &rp));
+  info->n = rp.best.n;
+  info->cliques = rp.best.cliques;
+  info->density = rp.best.density;
+  info->m = (uint32_t)rp.best.edges;
   // Upper bound from the loads the T passes added: (r - r0) / T is a feasible
   // fractional assignment of the cliques (every pass gives each clique one
   // unit), and the bound of kCDensestNoAtom.c:352-369 needs the loads in

@@ -118,6 +118,8 @@ kclpp_status ctx_check_err(kclpp_ctx *c);
 const HostDag &graph_dag(const kclpp_graph *g);
 const uint64_t *graph_dev_offsets(const kclpp_graph *g);
 const uint32_t *graph_dev_cols(const kclpp_graph *g);
+// Every vertex with an out-edge, by decreasing out-degree (unsharded graphs).
+const uint32_t *graph_dev_count_roots(const kclpp_graph *g);
 const uint4 *graph_dev_bit_rows(const kclpp_graph *g);  // nullptr: none
 const uint32_t *graph_dev_bits(const kclpp_graph *g);
 int graph_device(const kclpp_graph *g);
