@@ -1022,6 +1022,30 @@ struct TinyStream {
   }
 };
 
+// Bits over a group of ng rows (offsets ro[0..ng), 16-byte aligned, zero up to a
+// multiple of 4; members [a, a + ng) of a list): bit g set iff the group's row
+// g holds the member of local id `id` and list position j.  The rows are read
+// word by word at its bit.  A row ends at its own word; what is read beyond
+// belongs to ids above the row's and is masked off (only rows after j hold it).
+__device__ __forceinline__ uint32_t column_bits(const uint32_t *rows, const uint32_t *ro, uint32_t id, int j, int a,
+                                                int ng) {
+  const uint32_t *col = rows + (id >> 5);
+  const uint32_t bit = 1u << (id & 31);
+  uint32_t t = 0;
+  for (int g = 0; g < ng; g += 4) {
+    const uint4 o = *reinterpret_cast<const uint4 *>(ro + g);
+    uint32_t x = 0;
+    if (col[o.x] & bit) x |= 1u;
+    if (col[o.y] & bit) x |= 2u;
+    if (col[o.z] & bit) x |= 4u;
+    if (col[o.w] & bit) x |= 8u;
+    t |= x << g;
+  }
+  const int lo = j + 1 - a;
+  const uint32_t gmask = ng < 32 ? (1u << ng) - 1u : 0xffffffffu;
+  return t & (lo <= 0 ? gmask : (lo >= 32 ? 0u : gmask & (0xffffffffu << lo)));
+}
+
 // The members of P (lane w: word w), ascending, into list.
 __device__ __forceinline__ int list_members(uint32_t P, uint16_t *list, int lane) {
   const uint32_t lt = lanemask_lt();
@@ -1077,27 +1101,6 @@ struct PairLevel {
     } else {
       val[id] = v;
     }
-  }
-
-  // Bits of T for the member of id (list position j): the group's rows, read
-  // word by word at its bit.  A row ends at its own word; what is read beyond
-  // belongs to ids above u and is masked off (only u's after i in P hold i).
-  __device__ __forceinline__ uint32_t column(uint32_t id, int j, int a, int ng) const {
-    const uint32_t *col = rows + (id >> 5);
-    const uint32_t bit = 1u << (id & 31);
-    uint32_t t = 0;
-    for (int g = 0; g < ng; g += 4) {
-      const uint4 o = *reinterpret_cast<const uint4 *>(ro() + g);
-      uint32_t x = 0;
-      if (col[o.x] & bit) x |= 1u;
-      if (col[o.y] & bit) x |= 2u;
-      if (col[o.z] & bit) x |= 4u;
-      if (col[o.w] & bit) x |= 8u;
-      t |= x << g;
-    }
-    const int lo = j + 1 - a;
-    const uint32_t gmask = ng < 32 ? (1u << ng) - 1u : 0xffffffffu;
-    return t & (lo <= 0 ? gmask : (lo >= 32 ? 0u : gmask & (0xffffffffu << lo)));
   }
 
   // A chain of one slot whose every candidate is in I with nothing between
@@ -1171,7 +1174,7 @@ struct PairLevel {
         ro()[lane] = off;
         if (in && low) sv()[gi] = make_uint2(v, S);
         __syncwarp();
-        uint32_t T = column(id, at, a, ng);
+        uint32_t T = column_bits(rows, ro(), id, at, a, ng);
         if (!low) T = 0;  // the others always fall
         uint32_t inc = (uint32_t)__popc(T & ~Lg);
         const uint32_t taken = inc;
@@ -1289,7 +1292,7 @@ struct PairLevel {
           const bool low = j < a + ng && v + S < c;
           uint32_t inc = 0;
           if (__any_sync(KCL_FULL, low)) {
-            uint32_t T = column(i < ni ? list()[j] : 0u, j, a, ng);
+            uint32_t T = column_bits(rows, ro(), i < ni ? list()[j] : 0u, j, a, ng);
             if (!low) T = 0;  // the others always fall
             inc = (uint32_t)__popc(T & ~Lg);
             taken += inc;
@@ -1775,6 +1778,51 @@ __device__ __forceinline__ void seq_streams_shared(uint32_t *next, int d, const 
   }
 }
 
+// A root's induced rows (MakeSubgraph's induced adjacency,
+// kCDensestNoAtom.c:104-113), one warp per row i: the members of list[0, i)
+// that are out-neighbours of list[i].  A member with a bitmap row is asked
+// about 32 earlier members at a time: word(i, w, hit), all lanes, the lane's
+// member being 32 w + lane; the others' out-lists are walked, a lane per
+// out-neighbour, and looked up in the table: pair(i, j) on the finding lane.
+// Latency bounds this phase (a row's offsets, its list and the look-ups are
+// dependent reads), and it was 42 to 68 % of a CTA's time once the streams were
+// cheap: walking every list with a binary search, the k = 3 wave passes of an
+// RMAT-17 graph took 6.0 ms, now 3.2; the k = 4 count of RMAT-18 4.1 -> 2.2 ms,
+// a Seq pass over the RMAT-18 core 1.36 -> 1.03 ms.
+template <typename Word, typename Pair>
+__device__ __forceinline__ void induce_rows(const PassArgs &a, const uint32_t *list, int d, const uint32_t *tab, int tb,
+                                            int wid, int nwarps, int lane, Word &&word, Pair &&pair) {
+  for (int r0 = wid; r0 < d; r0 += nwarps * 32) {
+    // this warp's next 32 rows: r0, r0 + nwarps, ...
+    const int ri = r0 + nwarps * lane;
+    const uint4 br = ri < d ? bit_row(a, list[ri]) : make_uint4(kNoBitRow, 0u, 0u, 0u);
+    for (int q = 0, i = r0; q < 32 && i < d; ++q, i += nwarps) {
+      const uint32_t bo = __shfl_sync(KCL_FULL, br.x, q), bf = __shfl_sync(KCL_FULL, br.y, q);
+      const uint32_t bs = __shfl_sync(KCL_FULL, br.z, q);
+      if (i == 0) continue;
+      if (bo != kNoBitRow) {
+        const int nw = (i + 31) >> 5;
+#pragma unroll 4
+        for (int w = 0; w < nw; ++w) {
+          const int j = (w << 5) | lane;
+          word(i, w, j < i && bit_at(a, bo, bf, bs, list[j]));
+        }
+        continue;
+      }
+      const uint32_t x = list[i];
+      const uint32_t top = list[i - 1];
+      const uint64_t xe = a.off[x + 1];
+      for (uint64_t e = a.off[x] + lane; e < xe; e += 32) {
+        const uint32_t y = a.cols[e];
+        if (y > top) break;  // ascending: no later neighbour is in list[0, i)
+        const int j = tab_find(tab, tb, list, y);
+        if (j >= 0) pair(i, j);
+      }
+      __syncwarp();
+    }
+  }
+}
+
 // Work stealing: once the root list is exhausted, an idle CTA joins a root
 // whose sub-tasks (root edges or rows) are not all taken, rebuilds that root's
 // G_s and takes sub-tasks from the same global counter.  Every CTA publishes
@@ -1961,16 +2009,7 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
     if (K >= 3) {
       for (int i = tid; i < d; i += NW * 32) tab_insert(tab, tb, list[i], i);
       __syncthreads();
-      // Row i: N+(list[i]) ∩ N+(s) (MakeSubgraph's induced adjacency,
-      // kCDensestNoAtom.c:104-113), one warp per row.  A member with a bitmap
-      // row is asked about 32 earlier members at a time (a word of row i per
-      // ballot); the others' out-lists are walked, a lane per out-neighbour,
-      // and looked up in the table.  Latency bounds this phase (a row's
-      // offsets, its list and the look-ups are dependent reads), and it was 42
-      // to 68 % of a CTA's time once the streams were cheap: walking every
-      // list with a binary search, the k = 3 wave passes of an RMAT-17 graph
-      // took 6.0 ms, now 3.2; the k = 4 count of RMAT-18 4.1 -> 2.2 ms, a Seq
-      // pass over the RMAT-18 core 1.36 -> 1.03 ms.
+      // Row i: N+(list[i]) ∩ N+(s).
       auto put = [&](int i, int j) {  // j, before i, is its neighbour
         if constexpr (MODE == MODE_SEQ) {
           atomicOr(&rows[(size_t)tri_off((uint32_t)i) + (j >> 5)], 1u << (j & 31));
@@ -1983,45 +2022,21 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
           atomicOr(&rows[(size_t)lo * W + (hi >> 5)], 1u << (hi & 31));
         }
       };
-      for (int r0 = wid; r0 < d; r0 += NW * 32) {
-        // this warp's next 32 rows: r0, r0 + NW, ...
-        const int ri = r0 + NW * lane;
-        const uint4 br = ri < d ? bit_row(a, list[ri]) : make_uint4(kNoBitRow, 0u, 0u, 0u);
-        for (int q = 0, i = r0; q < 32 && i < d; ++q, i += NW) {
-          const uint32_t bo = __shfl_sync(KCL_FULL, br.x, q), bf = __shfl_sync(KCL_FULL, br.y, q);
-          const uint32_t bs = __shfl_sync(KCL_FULL, br.z, q);
-          if (i == 0) continue;
-          if (bo != kNoBitRow) {
-            const int nw = (i + 31) >> 5;
-#pragma unroll 4
-            for (int w = 0; w < nw; ++w) {
-              const int j = (w << 5) | lane;
-              const bool hit = j < i && bit_at(a, bo, bf, bs, list[j]);
-              if constexpr (MODE == MODE_SEQ) {
-                const uint32_t m = __ballot_sync(KCL_FULL, hit);
-                if (lane == 0) rows[(size_t)tri_off((uint32_t)i) + w] = m;
-              } else if constexpr (MODE == MODE_COUNT) {
-                const uint32_t m = __ballot_sync(KCL_FULL, hit);
-                if (lane == 0 && m) atomicOr(&rows[(size_t)i * W + w], m);
-                if (hit) atomicOr(&rows[(size_t)j * W + (i >> 5)], 1u << (i & 31));
-              } else if (hit) {
-                put(i, j);
-              }
+      induce_rows(
+          a, list, d, tab, tb, wid, NW, lane,
+          [&](int i, int w, bool hit) {
+            if constexpr (MODE == MODE_SEQ) {
+              const uint32_t m = __ballot_sync(KCL_FULL, hit);
+              if (lane == 0) rows[(size_t)tri_off((uint32_t)i) + w] = m;
+            } else if constexpr (MODE == MODE_COUNT) {
+              const uint32_t m = __ballot_sync(KCL_FULL, hit);
+              if (lane == 0 && m) atomicOr(&rows[(size_t)i * W + w], m);
+              if (hit) atomicOr(&rows[(size_t)((w << 5) | lane) * W + (i >> 5)], 1u << (i & 31));
+            } else if (hit) {
+              put(i, (w << 5) | lane);
             }
-            continue;
-          }
-          const uint32_t x = list[i];
-          const uint32_t top = list[i - 1];
-          const uint64_t xe = a.off[x + 1];
-          for (uint64_t e = a.off[x] + lane; e < xe; e += 32) {
-            const uint32_t y = a.cols[e];
-            if (y > top) break;  // ascending: no later neighbour is in list[0, i)
-            const int j = tab_find(tab, tb, list, y);
-            if (j >= 0) put(i, j);
-          }
-          __syncwarp();
-        }
-      }
+          },
+          put);
       __syncthreads();
     }
     if constexpr (MODE == MODE_SEQ) {
