@@ -70,15 +70,21 @@ static cudaEvent_t take_event(kclpp_ctx *c) {
   return e;
 }
 
-// Scheduler words of a pass: root counters of up to 5 launch groups, then one
-// stealing registry (kActiveSlots words) per group.
+// Scheduler words of a pass: the launch groups' root counters first.
 constexpr size_t kWorkActive = 32;
-constexpr size_t kWorkWords = kWorkActive + 5 * (size_t)kActiveSlots;
+// Words of it: then one sub-task counter per root and one stealing registry
+// per launch group, all zero at the start of a pass.
+constexpr size_t kMaxGroups = 6;
+static inline size_t work_words(uint32_t roots, size_t groups) {
+  return kWorkActive + roots + groups * (size_t)kActiveSlots;
+}
 
 struct TierInfo {
   int tier;
   int bucket;  // 0..3: the M1, M2, M3 and L root groups (kclpp_schedule.seq_warps); -1: tier S
   uint32_t offset, count, dmax;
+  uint32_t over32 = 0;  // tier S: roots of out-degree above 32 (the first ones)
+  uint32_t dmax32 = 0;  // tier S: the largest out-degree of the others
 };
 
 struct kclpp_graph {
@@ -107,11 +113,9 @@ struct kclpp_graph {
   unsigned long long *d_a = nullptr, *d_b = nullptr;
   double *d_rho = nullptr;
   uint32_t *d_level = nullptr;
-  uint32_t *d_work = nullptr;   // [0,16): root counters per tier; from kWorkActive: the
-                                // stealing registries, kActiveSlots words per tier
-  uint32_t *d_task = nullptr;   // per-root sub-task counters (tiers M, L)
+  uint32_t *d_work = nullptr;   // scheduler words (work_words)
   uint32_t num_roots = 0;
-  uint32_t task_cap = 0;
+  size_t work_cap = 0;
   unsigned long long *d_scalar = nullptr;
   uint32_t *d_slab = nullptr;
   uint64_t slab_words = 0;
@@ -164,6 +168,16 @@ __global__ void k_bit_rows(const uint64_t *off, const uint32_t *cols, const uint
       atomicOr(bits + r.x + (t >> 5), 1u << (t & 31));
     }
   }
+}
+
+// Start of a pass: the output zeroed or copied from in, the scheduler's words zeroed.
+__global__ void k_begin(unsigned long long *out, const unsigned long long *in, uint32_t n, uint32_t *words,
+                        uint64_t nwords) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  const uint64_t first = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (out)
+    for (uint64_t i = first; i < n; i += stride) out[i] = in ? in[i] : 0ull;
+  for (uint64_t i = first; i < nwords; i += stride) words[i] = 0;
 }
 
 inline int blocks_for(uint64_t n, int t = 256) { return (int)std::max<uint64_t>(1, (n + t - 1) / t); }
@@ -231,6 +245,10 @@ static kclpp_status build_schedule(kclpp_ctx *c, kclpp_graph *g) {
     const uint32_t da = deg(a), db = deg(b);
     return da != db ? da > db : a < b;
   };
+  auto split32 = [&](const std::vector<uint32_t> &v, TierInfo &t) {
+    while (t.over32 < t.count && deg(v[t.over32]) > 32) ++t.over32;
+    t.dmax32 = t.over32 < t.count ? deg(v[t.over32]) : 0;
+  };
   std::vector<uint32_t> all;
   bool any_l = false;
   uint32_t mx = 0;
@@ -262,6 +280,7 @@ static kclpp_status build_schedule(kclpp_ctx *c, kclpp_graph *g) {
       t.offset = (uint32_t)all.size();
       t.count = (uint32_t)v.size();
       t.dmax = deg(v.front());
+      if (tier == 0) split32(v, t);
       all.insert(all.end(), v.begin(), v.end());
       g->tiers[sch].push_back(t);
     };
@@ -306,6 +325,7 @@ static kclpp_status build_schedule(kclpp_ctx *c, kclpp_graph *g) {
         t.offset = (uint32_t)all.size();
         t.count = (uint32_t)v.size();
         t.dmax = deg(v.front());
+        if (tier == 0) split32(v, t);
         all.insert(all.end(), v.begin(), v.end());
         tw.push_back(t);
       };
@@ -320,14 +340,14 @@ static kclpp_status build_schedule(kclpp_ctx *c, kclpp_graph *g) {
   KCL_TRY(dalloc(&g->d_roots, all.size()));
   if (!all.empty())
     KCL_CUDA(cudaMemcpyAsync(g->d_roots, all.data(), all.size() * 4, cudaMemcpyHostToDevice, c->stream));
-  KCL_TRY(dalloc(&g->d_work, kWorkWords));
-  if (g->num_roots > g->task_cap) {  // the counters must cover every root of the schedule
-    cudaFree(g->d_task);
-    g->d_task = nullptr;
-    g->task_cap = 0;
+  const size_t words = work_words(g->num_roots, kMaxGroups);
+  if (words > g->work_cap) {  // the counters must cover every root of the schedule
+    cudaFree(g->d_work);
+    g->d_work = nullptr;
+    g->work_cap = 0;
   }
-  KCL_TRY(dalloc(&g->d_task, g->num_roots));
-  g->task_cap = std::max(g->task_cap, std::max<uint32_t>(g->num_roots, 1));
+  KCL_TRY(dalloc(&g->d_work, words));
+  g->work_cap = std::max(g->work_cap, words);
   if (any_l) {
     g->slab_ctas = c->num_sms;
     const uint64_t W = (kTierLMax + 31) / 32;
@@ -403,29 +423,93 @@ static void free_graph_dev(kclpp_graph *g) {
   cudaFree(g->d_order); cudaFree(g->d_best);
   cudaFree(g->d_off); cudaFree(g->d_cols); cudaFree(g->d_src); cudaFree(g->d_roots);
   cudaFree(g->d_a); cudaFree(g->d_b); cudaFree(g->d_rho); cudaFree(g->d_level);
-  cudaFree(g->d_work); cudaFree(g->d_task); cudaFree(g->d_scalar); cudaFree(g->d_slab);
+  cudaFree(g->d_work); cudaFree(g->d_scalar); cudaFree(g->d_slab);
 }
 
 // Where a pass runs: its stream and its scheduler counters.  Concurrent passes
 // (the batch's k values) each need their own counters.
 struct Exec {
   cudaStream_t st;
-  uint32_t *work;  // kWorkWords words
-  uint32_t *task;  // one per root
+  uint32_t *work;  // work_words(roots, kMaxGroups)
 };
 
+// The launches of one pass at clique size k, from the schedule's groups.
+//  * Seq, k <= 4: a CTA-per-root group whose roots have at most 32 members
+//    joins the warp-per-root group that follows it (one launch, lanes enough
+//    for the root edges): 20,000 vertices of out-degree <= 29 at k = 4, 149 us
+//    a pass apart, 89 together; 10,000 with 632 such roots 53 and 46.  From
+//    k = 5 on a lane's stream is long, and the CTA stays the better one.
+//  * Counting, k >= 5: warp-per-root roots above 32 members, whose rows a lane
+//    counts alone, go to a CTA: a core of out-degree 120 at k = 5, 424 us a Sim
+//    pass with the warp, 228 with the CTA; at k = 4 there is no difference.
+static std::vector<TierInfo> launch_plan(const std::vector<TierInfo> &tiers, int mode, int k) {
+  std::vector<TierInfo> plan;
+  for (TierInfo t : tiers) {
+    const TierInfo *prev = plan.empty() ? nullptr : &plan.back();
+    if (mode == dev::MODE_SEQ && k <= 4 && t.tier == 1 && t.dmax <= 32) {
+      t.tier = 0;
+      t.bucket = -1;
+    } else if (mode == dev::MODE_SEQ && k <= 4 && t.tier == 0 && prev && prev->tier == 0 &&
+               prev->offset + prev->count == t.offset) {
+      plan.back().count += t.count;
+      continue;
+    } else if (mode != dev::MODE_SEQ && k >= 5 && t.tier == 0 && t.over32) {
+      TierInfo hi = t;
+      hi.tier = 1;
+      hi.bucket = 0;
+      hi.count = t.over32;
+      plan.push_back(hi);
+      if (t.count == t.over32) continue;
+      t.offset += t.over32;
+      t.count -= t.over32;
+      t.dmax = t.dmax32;
+    }
+    plan.push_back(t);
+  }
+  return plan;
+}
+
+// Smallest root that idle CTAs join.  Joining means building the root's rows
+// again, which pays where its streams cost more: never at k = 3 (RMAT-17: 680
+// us a pass without, 912 with), from 128 members at k = 4 (a core of out-degree
+// 371: 660 us without, 482 with; 60,000 vertices, out-degree <= 128: 240 and
+// 290), from 32 beyond (a core of out-degree 120 at k = 5: 1656 and 779).
+static uint32_t steal_from(int mode, int k) {
+  return mode != dev::MODE_SEQ ? 0u : k == 3 ? UINT32_MAX : k == 4 ? 129u : 33u;
+}
+
+// What a pass's output holds before its kernels add to it.
+enum class Begin { keep, zero, copy };  // copy: of a.r_in
+
 // Launch every tier of one mode.
-static kclpp_status run_tiers(kclpp_ctx *c, kclpp_graph *g, int mode, int k, dev::PassArgs a,
+static kclpp_status run_tiers(kclpp_ctx *c, kclpp_graph *g, int mode, int k, dev::PassArgs a, Begin begin,
                               const Exec *ex = nullptr, int wave = -1) {
   const int sch = mode == dev::MODE_SEQ ? 1 : 0;
   const bool wv = mode == dev::MODE_SEQ && wave >= 0;
-  const std::vector<TierInfo> &tiers = wv ? g->wave_tiers[wave] : g->tiers[sch];
+  const std::vector<TierInfo> tiers = launch_plan(wv ? g->wave_tiers[wave] : g->tiers[sch], mode, k);
   const uint32_t base = wv ? g->wave_base[wave] : g->sched_base[sch];
+  const Exec E = ex ? *ex : Exec{c->stream, g->d_work};
+  // Work stealing pays off for the Seq chains (long, uneven root edges); the
+  // counting kernels finish their roots quickly and by default do not steal.
+  const uint32_t steal_min = steal_from(mode, k);
+  bool steal = false;
+  for (const TierInfo &t : tiers)
+    steal |= t.tier > 0 && t.dmax >= steal_min && (mode == dev::MODE_SEQ ? g->sp.steal_seq : g->sp.steal_count) != 0;
+  a.steal_min = steal_min;
+  // One launch prepares the output and the scheduler's words (the copy and
+  // three memsets of each pass took ~8 us of a small graph's 76).
+  const uint32_t n = g->dag.n;
+  const uint64_t words = tiers.empty() ? 0 : work_words(g->num_roots, steal ? tiers.size() : 0);
+  const uint64_t most = std::max<uint64_t>(begin == Begin::keep ? 0 : n, words);
+  if (most) {
+    k_begin<<<(int)std::min<uint64_t>((most + 255) / 256, (uint64_t)c->num_sms * 8), 256, 0, E.st>>>(
+        begin == Begin::keep ? nullptr : a.out, begin == Begin::copy ? a.r_in : nullptr, n, E.work, words);
+    KCL_CUDA(cudaGetLastError());
+    c->launches++;
+  }
   if (tiers.empty()) return KCLPP_OK;
-  const Exec E = ex ? *ex : Exec{c->stream, g->d_work, g->d_task};
-  KCL_CUDA(cudaMemsetAsync(E.work, 0, kWorkActive * sizeof(uint32_t), E.st));
-  KCL_CUDA(cudaMemsetAsync(E.work + kWorkActive, 0xff, (kWorkWords - kWorkActive) * sizeof(uint32_t), E.st));
-  KCL_CUDA(cudaMemsetAsync(E.task, 0, (size_t)g->num_roots * sizeof(uint32_t), E.st));
+  uint32_t *const task = E.work + kWorkActive;
+  uint32_t *const registry = task + g->num_roots;
   a.off = g->d_off;
   a.cols = g->d_cols;
   a.err = c->d_err;
@@ -453,11 +537,8 @@ static kclpp_status run_tiers(kclpp_ctx *c, kclpp_graph *g, int mode, int k, dev
     tl.num_roots = t.count;
     tl.dmax = t.dmax;
     tl.work = E.work + i;
-    tl.task_next = E.task + (t.offset - base);
-    // Work stealing pays off for the Seq chains (long, uneven root edges); the
-    // counting kernels finish their roots quickly and by default do not steal.
-    const bool steal = mode == dev::MODE_SEQ ? g->sp.steal_seq != 0 : g->sp.steal_count != 0;
-    tl.active = steal ? E.work + kWorkActive + i * kActiveSlots : nullptr;
+    tl.task_next = task + (t.offset - base);
+    tl.active = steal && t.tier > 0 && t.dmax >= steal_min ? registry + i * kActiveSlots : nullptr;
     tl.num_sms = c->num_sms;
     tl.max_grid = t.tier == 2 ? g->slab_ctas : 0;
     tl.warps = t.bucket < 0 ? 0 : (int)(mode == dev::MODE_SEQ ? g->sp.seq_warps[t.bucket] : g->sp.count_warps[t.bucket]);
@@ -511,35 +592,34 @@ static kclpp_status seq_pass_dev(kclpp_ctx *c, kclpp_graph *g, int k, const unsi
   if (det_mode == KCLPP_SEQ_WAVES && g->wave_tiers.size() > 1 && in != out) {
     unsigned long long *src = const_cast<unsigned long long *>(in), *dst = out;
     for (size_t w = 0; w < g->wave_tiers.size(); ++w) {
-      KCL_CUDA(cudaMemcpyAsync(dst, src, (size_t)n * 8, cudaMemcpyDeviceToDevice, c->stream));
       dev::PassArgs a{};
       a.r_in = src;
       a.out = dst;
-      KCL_TRY(run_tiers(c, g, dev::MODE_SEQ, k, a, nullptr, (int)w));
+      KCL_TRY(run_tiers(c, g, dev::MODE_SEQ, k, a, Begin::copy, nullptr, (int)w));
       std::swap(src, dst);
     }
     if (src != out) KCL_CUDA(cudaMemcpyAsync(out, src, (size_t)n * 8, cudaMemcpyDeviceToDevice, c->stream));
     return KCLPP_OK;
   }
-  if (in != out) KCL_CUDA(cudaMemcpyAsync(out, in, (size_t)n * 8, cudaMemcpyDeviceToDevice, c->stream));
   dev::PassArgs a{};
   a.r_in = in;
   a.out = out;
   if (det_mode == KCLPP_SEQ_SHARED) {
+    if (in != out) KCL_CUDA(cudaMemcpyAsync(out, in, (size_t)n * 8, cudaMemcpyDeviceToDevice, c->stream));
     // One load vector, read and added to in place by every stream.
     a.r_in = out;
     a.shared_loads = 1;
+    return run_tiers(c, g, dev::MODE_SEQ, k, a, Begin::keep);
   }
-  return run_tiers(c, g, dev::MODE_SEQ, k, a);
+  return run_tiers(c, g, dev::MODE_SEQ, k, a, in != out ? Begin::copy : Begin::keep);
 }
 
 static kclpp_status sim_counts_dev(kclpp_ctx *c, kclpp_graph *g, int k, const double *rho, unsigned long long *cnt) {
-  KCL_CUDA(cudaMemsetAsync(cnt, 0, (size_t)g->dag.n * 8, c->stream));
   dev::PassArgs a{};
   a.key_kind = dev::KEY_SIM;
   a.rho = rho;
   a.out = cnt;
-  return run_tiers(c, g, dev::MODE_ORDER, k, a);
+  return run_tiers(c, g, dev::MODE_ORDER, k, a, Begin::zero);
 }
 
 static kclpp_status sim_pass_dev(kclpp_ctx *c, kclpp_graph *g, int k, uint32_t t, double *rho) {
@@ -556,12 +636,11 @@ static kclpp_status sim_pass_dev(kclpp_ctx *c, kclpp_graph *g, int k, uint32_t t
 static kclpp_status pava_dev(kclpp_ctx *c, kclpp_graph *g, int k, const uint32_t *level_dev,
                              unsigned long long *tent_dev) {
   const uint32_t n = g->dag.n;
-  KCL_CUDA(cudaMemsetAsync(g->d_a, 0, (size_t)n * 8, c->stream));
   dev::PassArgs a{};
   a.key_kind = dev::KEY_LEVEL;
   a.level = level_dev;
   a.out = g->d_a;
-  KCL_TRY(run_tiers(c, g, dev::MODE_ORDER, k, a));
+  KCL_TRY(run_tiers(c, g, dev::MODE_ORDER, k, a, Begin::zero));
   if (n) {
     k_scatter_level<<<blocks_for(n), 256, 0, c->stream>>>(tent_dev, g->d_a, level_dev, n);
     KCL_CUDA(cudaGetLastError());
@@ -810,17 +889,15 @@ kclpp_status kclpp_count_cliques(kclpp_ctx *c, const kclpp_graph *gc, int k, uin
   KCL_TRY(set_device(c));
   kclpp_graph *g = const_cast<kclpp_graph *>(gc);
   const uint32_t n = g->dag.n;
-  KCL_CUDA(cudaMemsetAsync(g->d_a, 0, (size_t)n * 8 + 8, c->stream));
   dev::PassArgs a{};
   a.out = g->d_a;
-  KCL_TRY(run_tiers(c, g, dev::MODE_COUNT, k, a));
+  KCL_TRY(run_tiers(c, g, dev::MODE_COUNT, k, a, Begin::zero));
+  std::vector<uint64_t> own(per_vertex ? 0 : n);
+  uint64_t *const h = per_vertex ? per_vertex : own.data();
+  if (n) KCL_CUDA(cudaMemcpyAsync(h, g->d_a, (size_t)n * 8, cudaMemcpyDeviceToHost, c->stream));
   KCL_TRY(check_err(c));
-  std::vector<uint64_t> h(n);
-  if (n) KCL_CUDA(cudaMemcpyAsync(h.data(), g->d_a, (size_t)n * 8, cudaMemcpyDeviceToHost, c->stream));
-  KCL_CUDA(cudaStreamSynchronize(c->stream));
   unsigned __int128 sum = 0;
-  for (uint64_t v : h) sum += v;
-  if (per_vertex && n) memcpy(per_vertex, h.data(), (size_t)n * 8);
+  for (uint32_t i = 0; i < n; ++i) sum += h[i];
   if (total) *total = (uint64_t)(sum / (unsigned)k);
   return KCLPP_OK;
 }
@@ -956,11 +1033,10 @@ kclpp_status kclpp_seq_delta_dev(kclpp_ctx *c, const kclpp_graph *gc, int k, con
   KCL_TRY(set_device(c));
   kclpp_graph *g = const_cast<kclpp_graph *>(gc);
   if (!g->dag.n) return KCLPP_OK;
-  KCL_CUDA(cudaMemsetAsync(delta_dev, 0, (size_t)g->dag.n * 8, c->stream));
   dev::PassArgs a{};
   a.r_in = (const unsigned long long *)r_dev;
   a.out = (unsigned long long *)delta_dev;
-  return run_tiers(c, g, dev::MODE_SEQ, k, a);
+  return run_tiers(c, g, dev::MODE_SEQ, k, a, Begin::zero);
 }
 
 kclpp_status kclpp_sim_counts_dev(kclpp_ctx *c, const kclpp_graph *gc, int k, const double *rho_dev, uint64_t *cnt_dev) {
@@ -1194,7 +1270,7 @@ struct BatchBranch {
   int k = 0;
   cudaStream_t st = nullptr;
   cudaEvent_t join = nullptr;
-  uint32_t *work = nullptr, *task = nullptr;
+  uint32_t *work = nullptr;
   unsigned long long *buf[2] = {nullptr, nullptr};  // Seq ping-pong, or Sim counts in buf[0]
   double *rho = nullptr;
   void *result = nullptr;  // device vector holding the branch's final r / rho
@@ -1216,7 +1292,7 @@ static void batch_release(kclpp_batch *b) {
   for (auto &x : b->br) {
     if (x.st) cudaStreamDestroy(x.st);
     if (x.join) cudaEventDestroy(x.join);
-    cudaFree(x.work); cudaFree(x.task); cudaFree(x.buf[0]); cudaFree(x.buf[1]); cudaFree(x.rho);
+    cudaFree(x.work); cudaFree(x.buf[0]); cudaFree(x.buf[1]); cudaFree(x.rho);
   }
   b->br.clear();
   if (b->exec) cudaGraphExecDestroy(b->exec);
@@ -1293,28 +1369,26 @@ static kclpp_status batch_record(kclpp_ctx *c, kclpp_batch *b, int kernel, uint3
   KCL_CUDA(cudaEventRecord(b->fork, c->stream));
   for (auto &x : b->br) {
     KCL_CUDA(cudaStreamWaitEvent(x.st, b->fork, 0));
-    const Exec E{x.st, x.work, x.task};
+    const Exec E{x.st, x.work};
     if (kernel == KCLPP_KERNEL_SEQ) {
       KCL_CUDA(cudaMemsetAsync(x.buf[0], 0, (size_t)n * 8, x.st));
       int cur = 0;
       for (uint32_t p = 0; p < passes; ++p) {
-        KCL_CUDA(cudaMemcpyAsync(x.buf[cur ^ 1], x.buf[cur], (size_t)n * 8, cudaMemcpyDeviceToDevice, x.st));
         dev::PassArgs a{};
         a.r_in = x.buf[cur];
         a.out = x.buf[cur ^ 1];
-        KCL_TRY(run_tiers(c, g, dev::MODE_SEQ, x.k, a, &E));
+        KCL_TRY(run_tiers(c, g, dev::MODE_SEQ, x.k, a, Begin::copy, &E));
         cur ^= 1;
       }
       x.result = x.buf[cur];
     } else {
       KCL_CUDA(cudaMemsetAsync(x.rho, 0, (size_t)n * 8, x.st));
       for (uint32_t p = 0; p < passes; ++p) {
-        KCL_CUDA(cudaMemsetAsync(x.buf[0], 0, (size_t)n * 8, x.st));
         dev::PassArgs a{};
         a.key_kind = dev::KEY_SIM;
         a.rho = x.rho;
         a.out = x.buf[0];
-        KCL_TRY(run_tiers(c, g, dev::MODE_ORDER, x.k, a, &E));
+        KCL_TRY(run_tiers(c, g, dev::MODE_ORDER, x.k, a, Begin::zero, &E));
         k_sim_update<<<blocks_for(n), 256, 0, x.st>>>(x.rho, x.buf[0], n, p + 1);
         KCL_CUDA(cudaGetLastError());
         c->launches++;
@@ -1351,8 +1425,7 @@ kclpp_status kclpp_batch_run(kclpp_ctx *c, kclpp_batch *b, int kernel, const int
       x.k = ks[i];
       KCL_CUDA(cudaStreamCreateWithFlags(&x.st, cudaStreamNonBlocking));
       KCL_CUDA(cudaEventCreateWithFlags(&x.join, cudaEventDisableTiming));
-      KCL_TRY(dalloc(&x.work, kWorkWords));
-      KCL_TRY(dalloc(&x.task, std::max<uint32_t>(g->num_roots, 1)));
+      KCL_TRY(dalloc(&x.work, work_words(g->num_roots, kMaxGroups)));
       KCL_TRY(dalloc(&x.buf[0], n));
       if (kernel == KCLPP_KERNEL_SEQ) KCL_TRY(dalloc(&x.buf[1], n));
       else KCL_TRY(dalloc(&x.rho, n));
@@ -1754,10 +1827,9 @@ kclpp_status kclpp_warm_features(kclpp_ctx *c, const kclpp_graph *gc, float *X_d
   // triangles and 4-cliques per vertex with the count kernels
   for (int k = 3; k <= 4; ++k) {
     unsigned long long *out = k == 3 ? g->d_a : g->d_b;
-    KCL_CUDA(cudaMemsetAsync(out, 0, (size_t)n * 8, c->stream));
     dev::PassArgs a{};
     a.out = out;
-    KCL_TRY(run_tiers(c, g, dev::MODE_COUNT, k, a));
+    KCL_TRY(run_tiers(c, g, dev::MODE_COUNT, k, a, Begin::zero));
   }
   KCL_TRY(kclpp_warm_features_dev(c, n, d_deg, d_core, (const uint64_t *)g->d_a, (const uint64_t *)g->d_b, X_dev));
   KCL_CUDA(cudaStreamSynchronize(c->stream));

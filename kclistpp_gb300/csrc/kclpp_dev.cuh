@@ -42,7 +42,7 @@ struct PassArgs {
   uint32_t dmax;                  // largest out-degree among them
   uint32_t *work;                 // root counter (zeroed before launch)
   uint32_t *task_next;            // tiers M, L: per-root sub-task counters (zeroed)
-  uint32_t *active;               // tiers M, L: one slot per CTA, the root it holds (nullptr: no stealing)
+  uint32_t *active;               // tiers M, L: one slot per CTA, the root it holds + 1 (zeroed; nullptr: no stealing)
   uint32_t *err;                  // status word
   int key_kind;                   // MODE_ORDER
   const double *rho;              // KEY_SIM
@@ -66,6 +66,7 @@ struct PassArgs {
   // of the pass, read by every stream when it starts and added to in place
   // when it closes.
   int shared_loads;
+  uint32_t steal_min;             // tiers M, L: smallest out-degree of a root that idle CTAs join
   // Bitmap rows of the vertices whose out-lists are dense in their id range
   // (nullptr: none): per vertex (first word in bits, id of its first bit, ids
   // covered; first word 0xffffffff and 0 ids: no row).

@@ -614,7 +614,7 @@ __host__ __device__ inline LayoutM layout_m(int mode, int k, uint32_t dmax, int 
   L.acc = at; if (mode == MODE_SEQ) at = align16(at + (size_t)(dmax + 1) * 8);
   L.rank = at; if (mode == MODE_ORDER) at = align16(at + (size_t)dmax * 2);
   L.inv = at; if (mode == MODE_ORDER) at = align16(at + (size_t)dmax * 2);
-  L.rel = at; if (mode == MODE_SEQ && k >= 4 && rows_in_smem) at = align16(at + (size_t)(dmax + 1) * 4);
+  L.rel = at; if (mode == MODE_SEQ && rows_in_smem) at = align16(at + (size_t)(dmax + 1) * 4);
   L.dl = at; if (mode == MODE_SEQ) at = align16(at + (size_t)nw * seq_warp_words(k, dmax, rows_in_smem) * 4);
   L.cbuf = at;
   if (mode != MODE_SEQ && (k == 4 || k == 5) && rows_in_smem) at = align16(at + (size_t)nw * cbuf_words(dmax) * 4);
@@ -826,7 +826,7 @@ __device__ __forceinline__ typename VA::T value_of(int x, const VA &va, int lane
 // communities), 15.0 -> 11.9 ms.  At most 40 registers at k = 4 (48 warps per
 // SM): at 80 (24 warps) the same pass took 2.16 ms.
 // Values of a root as 32-bit offsets from its smallest, capped here (the Seq
-// kernel at k >= 4 with rows in shared memory).
+// kernel with rows in shared memory).
 constexpr uint32_t kRelCap = 0x7ffffff0u;
 
 // A whole stream over at most 32 * S candidates, in registers: member i of C
@@ -1557,11 +1557,75 @@ __device__ __forceinline__ void for_members(const Bits<WPL> &C, int lane, F &&f)
   }
 }
 
+// A stream over the nc candidates C on the root's 32-bit values.  False, with
+// nothing done, when a prefix value it can reach comes near their cap (see
+// kRelCap), or its followed members outgrow the scratch.
+template <int K>
+__device__ __forceinline__ bool stream_on_rel(const Bits<1> &C, uint32_t nc, int g0, const uint32_t *rows,
+                                              const uint32_t *rel, uint32_t *cur, unsigned long long *acc,
+                                              uint32_t *pair, int lane, uint32_t *err) {
+  unsigned long long bound = 1;  // C(nc, K - 2): the stream's cliques at most
+#pragma unroll
+  for (uint32_t i = 0; i < (uint32_t)(K - 2); ++i) bound = bound * (nc - i) / (i + 1u);
+  const uint32_t c0 = rel[g0];
+  if (bound + 64 >= (unsigned long long)(kRelCap - c0)) return false;
+  uint32_t c = c0;
+  if constexpr (K == 3) {
+    // One chain: nothing reads a value twice, so the takers' units go straight
+    // to acc.
+    const uint32_t lt = lanemask_lt();
+    uint32_t nz = __ballot_sync(KCL_FULL, C.w[0] != 0);
+    while (nz) {
+      const int w = __ffs(nz) - 1;
+      nz &= nz - 1;
+      const uint32_t word = __shfl_sync(KCL_FULL, C.w[0], w);
+      const bool has = (word >> lane) & 1u;
+      const int v = (w << 5) | lane;
+      const uint32_t m = word_fixed_point(has ? (int)(rel[v] - c) : -1, lt);
+      if (has && !((m >> lane) & 1u)) shared_add(acc + v, 1u);
+      c += (uint32_t)__popc(m);
+    }
+  } else if (nc <= (K == 4 ? 32u : 64u)) {
+    // Two slots cost 64 column reads per member up front: k = 4, with one pair
+    // of levels per stream, has nothing to spread them over.
+    uint16_t *list = PairLevel<true>{nullptr, nullptr, nullptr, pair, lane}.list();
+    __syncwarp();
+    list_members(C.w[0], list, lane);
+    __syncwarp();
+    if (K == 4 || nc <= 32) {
+      TinyStream<1> ts;
+      ts.lane = lane;
+      c = ts.template run<K>(rows, list, (int)nc, rel, acc, c);
+    } else {
+      TinyStream<2> ts;
+      ts.lane = lane;
+      c = ts.template run<K>(rows, list, (int)nc, rel, acc, c);
+    }
+  } else if constexpr (K == 4) {
+    if (!PairLevel<true>{rows, const_cast<uint32_t *>(rel), acc, pair, lane}(C.w[0], c)) return false;
+  } else {
+    for_members<1>(C, lane, [&](int i) { cur[i] = rel[i]; });
+    const Vals32 va{cur};
+    c = seq_rec<K - 2, 1, Vals32, true, true>(C, c, rows, va, 0u, lane, err, pair);
+    __syncwarp();
+    for_members<1>(C, lane, [&](int i) {
+      const uint32_t delta = cur[i] - rel[i];
+      if (delta) shared_add(&acc[i], delta);
+    });
+  }
+  if (lane == 0 && c != c0) shared_add(&acc[g0], c - c0);
+  return true;
+}
+
+// A root's sub-task counter: sub-tasks taken below, CTAs that joined it above.
+constexpr int kTaskBits = 20;  // 2048 sub-tasks and one overshoot per warp of 2048 CTAs
+constexpr uint32_t kTaskMask = (1u << kTaskBits) - 1u;
+
 // Every root-edge stream of the current root, the warp taking streams from
 // the root's shared counter (largest candidate sets first); increments go to
 // the CTA's acc[] (kCDensestNoAtom.c:270-295 per root edge).
 //
-// k >= 4, rows in shared memory: the streams read rel, the root's values as
+// Rows in shared memory: the streams read rel, the root's values as
 // 32-bit offsets from the smallest of them capped at kRelCap; a stream whose
 // prefix value cannot reach the cap uses them (a capped member then lies above
 // every prefix value, so the cap changes no comparison).  Otherwise the
@@ -1581,63 +1645,17 @@ __device__ __forceinline__ void seq_streams(uint32_t *next, int d, const uint32_
                                             uint32_t *err) {
   for (;;) {
     int q = 0;
-    if (lane == 0) q = (int)atomicAdd(next, 1u);
+    if (lane == 0) q = (int)(atomicAdd(next, 1u) & kTaskMask);
     q = __shfl_sync(KCL_FULL, q, 0);
     if (q >= d) break;
     const int j = d - 1 - q;
     const Bits<WPL> C = load_row<WPL, true>(rows, j, 0, lane);
     if (!any_bits<WPL>(C)) continue;
     const int g0 = base[j] < base[d] ? j : d;  // kCDensestNoAtom.c:287
-    if constexpr (K >= 4 && WPL == 1) {
-      // The root's 32-bit values serve the stream when no prefix value it can
-      // reach comes near their cap (see kRelCap).
+    if constexpr (WPL == 1) {
       const uint32_t nc = __reduce_add_sync(KCL_FULL, (uint32_t)__popc(C.w[0]));
       if (nc < (uint32_t)(K - 2)) continue;
-      unsigned long long bound = 1;  // C(nc, K - 2): the stream's cliques at most
-#pragma unroll
-      for (uint32_t i = 0; i < (uint32_t)(K - 2); ++i) bound = bound * (nc - i) / (i + 1u);
-      const uint32_t c0 = rel[g0];
-      if (bound + 64 < (unsigned long long)(kRelCap - c0)) {
-        // Two slots cost 64 column reads per member up front: k = 4, with one
-        // pair of levels per stream, has nothing to spread them over.
-        constexpr int kTiny = K == 4 ? 32 : 64;
-        if (nc <= (uint32_t)kTiny) {
-          uint16_t *list = PairLevel<true>{nullptr, nullptr, nullptr, pair, lane}.list();
-          __syncwarp();
-          list_members(C.w[0], list, lane);
-          __syncwarp();
-          uint32_t c1;
-          if (K == 4 || nc <= 32) {
-            TinyStream<1> ts;
-            ts.lane = lane;
-            c1 = ts.template run<K>(rows, list, (int)nc, rel, acc, c0);
-          } else {
-            TinyStream<2> ts;
-            ts.lane = lane;
-            c1 = ts.template run<K>(rows, list, (int)nc, rel, acc, c0);
-          }
-          if (lane == 0 && c1 != c0) shared_add(&acc[g0], c1 - c0);
-          continue;
-        }
-        if constexpr (K == 4) {
-          uint32_t c = c0;
-          if (PairLevel<true>{rows, const_cast<uint32_t *>(rel), acc, pair, lane}(C.w[0], c)) {
-            if (lane == 0 && c != c0) shared_add(&acc[g0], c - c0);
-            continue;
-          }
-        } else {
-          for_members<1>(C, lane, [&](int i) { cur[i] = rel[i]; });
-          const Vals32 va{cur};
-          const uint32_t c1 = seq_rec<K - 2, 1, Vals32, true, true>(C, c0, rows, va, 0u, lane, err, pair);
-          __syncwarp();
-          for_members<1>(C, lane, [&](int i) {
-            const uint32_t delta = cur[i] - rel[i];
-            if (delta) shared_add(&acc[i], delta);
-          });
-          if (lane == 0 && c1 != c0) shared_add(&acc[g0], c1 - c0);
-          continue;
-        }
-      }
+      if (stream_on_rel<K>(C, nc, g0, rows, rel, cur, acc, pair, lane, err)) continue;
     }
     bool r32 = false;
     unsigned long long off = 0, cap = 0;
@@ -1730,7 +1748,7 @@ __device__ __forceinline__ void seq_streams_shared(uint32_t *next, int d, const 
   };
   for (;;) {
     int q = 0;
-    if (lane == 0) q = (int)atomicAdd(next, 1u);
+    if (lane == 0) q = (int)(atomicAdd(next, 1u) & kTaskMask);
     q = __shfl_sync(KCL_FULL, q, 0);
     if (q >= d) break;
     const int j = d - 1 - q;
@@ -1826,29 +1844,48 @@ __device__ __forceinline__ void induce_rows(const PassArgs &a, const uint32_t *l
 // Work stealing: once the root list is exhausted, an idle CTA joins a root
 // whose sub-tasks (root edges or rows) are not all taken, rebuilds that root's
 // G_s and takes sub-tasks from the same global counter.  Every CTA publishes
-// the root it holds in its slot of a.active, so a thief looks at the roots in
-// progress only (one slot per CTA, scanned by one warp) and joins the one with
-// the most sub-tasks left.  Returns UINT32_MAX when none has kMinSteal left.
-constexpr uint32_t kMinSteal = 2;
+// the root it holds (plus one; 0: none) in its slot of a.active; the thief's
+// threads look at a slot each and the CTA joins the root with the most
+// sub-tasks left per CTA on it, if that is at least steal_quarters of its warps
+// -- below, rebuilding the rows costs more than the share saves.  A root's
+// counter holds the sub-tasks taken in its low kTaskBits and the CTAs that
+// joined above.  (One warp scanning, every CTA joining the root with most left:
+// a Seq pass over the RMAT-18 core took 858 us, now 482.)
+// Least share in quarters of the CTA's warps: a sub-task grows with k.
+template <int MODE, int K>
+constexpr uint32_t steal_quarters() { return MODE == MODE_SEQ && K >= 5 ? 1 : 4; }
 template <bool IDENT>
-__device__ __forceinline__ uint32_t find_victim(const PassArgs &a, int need, int lane) {
-  uint32_t best = 0, best_idx = UINT32_MAX;  // best = sub-tasks left (0: none)
-  for (uint32_t b = lane; b < gridDim.x; b += 32) {
-    const uint32_t idx = *(volatile uint32_t *)(a.active + b);
-    if (idx >= a.num_roots) continue;
+__device__ __forceinline__ uint32_t find_victim(const PassArgs &a, int need, uint32_t least, uint32_t *s_best,
+                                                uint32_t *s_who) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = (int)(blockDim.x >> 5);
+  uint32_t best = 0, best_idx = UINT32_MAX;
+  for (uint32_t b = tid; b < gridDim.x; b += blockDim.x) {
+    const uint32_t held = __ldcg(a.active + b);
+    if (held == 0 || held > a.num_roots) continue;
+    const uint32_t idx = held - 1;
     const uint32_t s = IDENT ? idx : a.roots[idx];
     const uint32_t d = a.list_off ? (uint32_t)(a.list_off[s + 1] - a.list_off[s]) : (uint32_t)(a.off[s + 1] - a.off[s]);
-    const uint32_t taken = *(volatile uint32_t *)(a.task_next + idx);
+    const uint32_t t = __ldcg(a.task_next + idx), taken = t & kTaskMask;
     const bool in_window = !IDENT || (d >= a.deg_lo && d <= a.deg_hi && d <= a.dmax);
-    if (in_window && (int)d >= need && taken + kMinSteal <= d && d - taken > best) {
-      best = d - taken;
+    if (!in_window || (int)d < need || d < a.steal_min || taken >= d) continue;
+    const uint32_t share = (d - taken) / ((t >> kTaskBits) + 2u);  // with its owner, those who joined, and this CTA
+    if (share >= least && share > best) {
+      best = share;
       best_idx = idx;
     }
   }
   const uint32_t top = __reduce_max_sync(KCL_FULL, best);
-  if (top == 0) return UINT32_MAX;
   const uint32_t who = __ballot_sync(KCL_FULL, best == top);
-  return __shfl_sync(KCL_FULL, best_idx, __ffs(who) - 1);
+  const uint32_t idx = __shfl_sync(KCL_FULL, best_idx, __ffs(who) - 1);
+  if (lane == 0) {
+    s_best[wid] = top;
+    s_who[wid] = idx;
+  }
+  __syncthreads();
+  const uint32_t mine = lane < nw ? s_best[lane] : 0u;
+  const uint32_t all = __reduce_max_sync(KCL_FULL, mine);
+  if (all == 0) return UINT32_MAX;
+  return s_who[__ffs(__ballot_sync(KCL_FULL, mine == all)) - 1];
 }
 
 // Register budget of a tier M / L kernel, as CTAs of the widest launch that
@@ -1879,7 +1916,7 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
   uint32_t *rel = reinterpret_cast<uint32_t *>(smem_raw + lay.rel);
   uint32_t *cbuf = reinterpret_cast<uint32_t *>(smem_raw + lay.cbuf) + (size_t)wid * cbuf_words(a.dmax);
 
-  __shared__ uint32_t s_idx;
+  __shared__ uint32_t s_idx, s_best[32], s_who[32];
   __shared__ int s_tau;
   __shared__ unsigned long long s_sum;
   __shared__ unsigned long long s_off;  // Seq: the root's smallest value
@@ -1896,27 +1933,28 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
     __syncthreads();
     return warp_min_u64(lane < NW ? s_min[lane] : ~0ull);
   };
-  bool stealing = false;  // warp 0's view (uniform across its lanes)
+  bool stealing = false;
   __syncthreads();
   for (;;) {
-    if (wid == 0) {
-      uint32_t idx = UINT32_MAX;
-      if (!stealing) {
-        if (lane == 0) idx = atomicAdd(a.work, 1u);
-        idx = __shfl_sync(KCL_FULL, idx, 0);
-        if (idx >= a.num_roots) stealing = true;
-      }
-      if (stealing) idx = a.active ? find_victim<IDENT>(a, K - 1, lane) : UINT32_MAX;
-      if (lane == 0) {
-        s_idx = idx;
-        s_tau = 0;
-        s_sum = 0;
-        if (a.active && idx != UINT32_MAX) a.active[blockIdx.x] = idx;  // visible to thieves
-      }
+    uint32_t idx;
+    if (tid == 0) {
+      if (!stealing) s_idx = atomicAdd(a.work, 1u);
+      s_tau = 0;
+      s_sum = 0;
     }
-    __syncthreads();
-    const uint32_t idx = s_idx;
-    if (idx == UINT32_MAX) break;
+    if (!stealing) {
+      __syncthreads();
+      idx = s_idx;
+      stealing = idx >= a.num_roots;
+    }
+    if (stealing) {
+      if (!a.active) break;
+      const uint32_t least = ((uint32_t)NW * steal_quarters<MODE, K>() + 3u) / 4u;
+      idx = find_victim<IDENT>(a, K - 1, least > 2u ? least : 2u, s_best, s_who);
+      if (idx == UINT32_MAX) break;
+      if (tid == 0) atomicAdd(a.task_next + idx, 1u << kTaskBits);
+    }
+    if (tid == 0 && a.active) a.active[blockIdx.x] = idx + 1;  // visible to thieves
     uint32_t *next = a.task_next + idx;  // root's sub-task counter, shared by every CTA on it
     const uint32_t s = IDENT ? idx : a.roots[idx];
     uint64_t o;
@@ -1978,7 +2016,7 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
           base[i] = v;
           mn = v < mn ? v : mn;
         }
-        if constexpr (K >= 4 && ROWS_IN_SMEM) {
+        if constexpr (ROWS_IN_SMEM) {
           const unsigned long long off = cta_min(mn);
           for (int i = tid; i <= d; i += NW * 32) {
             const unsigned long long v = base[i] - off;
@@ -2059,7 +2097,7 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
       unsigned long long mine = 0;
       for (;;) {
         int p = 0;
-        if (lane == 0) p = (int)atomicAdd(next, 1u);
+        if (lane == 0) p = (int)(atomicAdd(next, 1u) & kTaskMask);
         p = __shfl_sync(KCL_FULL, p, 0);
         if (p >= d) break;
         const Bits<WPL> P = load_row<WPL>(rows, p, W, lane);
@@ -2102,7 +2140,7 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
         if constexpr (IDENT && MODE == MODE_COUNT) atomicAdd(a.total, s_sum);
       }
     }
-    if (tid == 0 && a.active) a.active[blockIdx.x] = UINT32_MAX;
+    if (tid == 0 && a.active) a.active[blockIdx.x] = 0;
     __syncthreads();
   }
 }

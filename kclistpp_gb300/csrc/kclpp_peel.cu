@@ -69,10 +69,9 @@ struct PeelRecount {
   uint32_t *d_lcols = nullptr;
   unsigned long long *d_w = nullptr;
   uint32_t *d_roots = nullptr;
-  uint32_t *d_task = nullptr;
-  uint32_t *d_work = nullptr;
+  uint32_t *d_work = nullptr;  // root counters, the two registries, then the sub-task counters
   uint32_t *d_slab = nullptr;
-  size_t cap_loff = 0, cap_lcols = 0, cap_w = 0, cap_roots = 0, cap_task = 0;
+  size_t cap_loff = 0, cap_lcols = 0, cap_w = 0, cap_roots = 0, cap_work = 0;
   uint64_t slab_words = 0;
   int slab_ctas = 0;
   // pinned staging
@@ -89,11 +88,6 @@ kclpp_status peel_recount_create(kclpp_ctx *c, const kclpp_graph *g, int k, Peel
   P->ctx = c;
   P->g = g;
   P->k = k;
-  cudaError_t e = cudaMalloc((void **)&P->d_work, (kPeelWorkHeader + 2 * kRegistryWords) * sizeof(uint32_t));
-  if (e != cudaSuccess) {
-    delete P;
-    return set_error(KCLPP_ERR_NOMEM, "peel recount: %s", cudaGetErrorString(e));
-  }
   *out = P;
   return KCLPP_OK;
 }
@@ -101,7 +95,7 @@ kclpp_status peel_recount_create(kclpp_ctx *c, const kclpp_graph *g, int k, Peel
 void peel_recount_free(PeelRecount *P) {
   if (!P) return;
   cudaFree(P->d_loff); cudaFree(P->d_lcols); cudaFree(P->d_w); cudaFree(P->d_roots);
-  cudaFree(P->d_task); cudaFree(P->d_work); cudaFree(P->d_slab);
+  cudaFree(P->d_work); cudaFree(P->d_slab);
   cudaFreeHost(P->h_loff); cudaFreeHost(P->h_lcols); cudaFreeHost(P->h_w); cudaFreeHost(P->h_roots);
   delete P;
 }
@@ -138,7 +132,7 @@ kclpp_status peel_recount_run(PeelRecount *P, uint32_t nroots, const uint64_t *l
   PCUDA(grow_dev(&P->d_lcols, &P->cap_lcols, (size_t)total));
   PCUDA(grow_dev(&P->d_w, &P->cap_w, (size_t)total));
   PCUDA(grow_dev(&P->d_roots, &P->cap_roots, nr));
-  PCUDA(grow_dev(&P->d_task, &P->cap_task, nr));
+  PCUDA(grow_dev(&P->d_work, &P->cap_work, kPeelWorkHeader + 2 * kRegistryWords + nr));
   if (!grp[0].empty() && !P->d_slab) {
     P->slab_ctas = ctx_sms(c);
     P->slab_words = (uint64_t)kTierLMax * ((kTierLMax + 31) / 32);
@@ -154,9 +148,8 @@ kclpp_status peel_recount_run(PeelRecount *P, uint32_t nroots, const uint64_t *l
   PCUDA(cudaMemcpyAsync(P->d_loff, P->h_loff, ((size_t)nroots + 1) * 8, cudaMemcpyHostToDevice, st));
   PCUDA(cudaMemcpyAsync(P->d_lcols, P->h_lcols, (size_t)total * 4, cudaMemcpyHostToDevice, st));
   PCUDA(cudaMemcpyAsync(P->d_roots, P->h_roots, nr * 4, cudaMemcpyHostToDevice, st));
-  PCUDA(cudaMemsetAsync(P->d_work, 0, kPeelWorkHeader * sizeof(uint32_t), st));
-  PCUDA(cudaMemsetAsync(P->d_work + kPeelWorkHeader, 0xff, 2 * kRegistryWords * sizeof(uint32_t), st));
-  PCUDA(cudaMemsetAsync(P->d_task, 0, nr * sizeof(uint32_t), st));
+  PCUDA(cudaMemsetAsync(P->d_work, 0, (kPeelWorkHeader + 2 * kRegistryWords + nr) * sizeof(uint32_t), st));
+  uint32_t *const d_task = P->d_work + kPeelWorkHeader + 2 * kRegistryWords;
   dev::PassArgs a{};
   a.off = graph_dev_offsets(P->g);
   a.cols = graph_dev_cols(P->g);
@@ -179,7 +172,7 @@ kclpp_status peel_recount_run(PeelRecount *P, uint32_t nroots, const uint64_t *l
     tl.num_roots = (uint32_t)v.size();
     tl.dmax = (uint32_t)(loff[v.front() + 1] - loff[v.front()]);
     tl.work = P->d_work + t;
-    tl.task_next = P->d_task + at;
+    tl.task_next = d_task + at;
     tl.active = t < 2 ? P->d_work + kPeelWorkHeader + (size_t)t * kRegistryWords : nullptr;
     tl.num_sms = ctx_sms(c);
     tl.max_grid = t == 0 ? P->slab_ctas : 0;
