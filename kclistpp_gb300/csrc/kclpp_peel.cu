@@ -65,21 +65,17 @@ struct PeelRecount {
   const kclpp_graph *g = nullptr;
   int k = 0;
   // device
-  uint64_t *d_loff = nullptr;
-  uint32_t *d_lcols = nullptr;
+  unsigned char *d_in = nullptr;  // list offsets, roots, lists: one copy a batch
   unsigned long long *d_w = nullptr;
-  uint32_t *d_roots = nullptr;
   uint32_t *d_work = nullptr;  // root counters, the two registries, then the sub-task counters
   uint32_t *d_slab = nullptr;
-  size_t cap_loff = 0, cap_lcols = 0, cap_w = 0, cap_roots = 0, cap_work = 0;
+  size_t cap_in = 0, cap_w = 0, cap_work = 0;
   uint64_t slab_words = 0;
   int slab_ctas = 0;
   // pinned staging
-  uint64_t *h_loff = nullptr;
-  uint32_t *h_lcols = nullptr;
+  unsigned char *h_in = nullptr;
   unsigned long long *h_w = nullptr;
-  uint32_t *h_roots = nullptr;
-  size_t hcap_loff = 0, hcap_lcols = 0, hcap_w = 0, hcap_roots = 0;
+  size_t hcap_in = 0, hcap_w = 0;
 };
 
 kclpp_status peel_recount_create(kclpp_ctx *c, const kclpp_graph *g, int k, PeelRecount **out) {
@@ -94,9 +90,8 @@ kclpp_status peel_recount_create(kclpp_ctx *c, const kclpp_graph *g, int k, Peel
 
 void peel_recount_free(PeelRecount *P) {
   if (!P) return;
-  cudaFree(P->d_loff); cudaFree(P->d_lcols); cudaFree(P->d_w); cudaFree(P->d_roots);
-  cudaFree(P->d_work); cudaFree(P->d_slab);
-  cudaFreeHost(P->h_loff); cudaFreeHost(P->h_lcols); cudaFreeHost(P->h_w); cudaFreeHost(P->h_roots);
+  cudaFree(P->d_in); cudaFree(P->d_w); cudaFree(P->d_work); cudaFree(P->d_slab);
+  cudaFreeHost(P->h_in); cudaFreeHost(P->h_w);
   delete P;
 }
 
@@ -124,30 +119,26 @@ kclpp_status peel_recount_run(PeelRecount *P, uint32_t nroots, const uint64_t *l
     nr += v.size();
   }
   if (nr == 0) return KCLPP_OK;
-  PCUDA(grow_host(&P->h_loff, &P->hcap_loff, (size_t)nroots + 1));
-  PCUDA(grow_host(&P->h_lcols, &P->hcap_lcols, (size_t)total));
+  const size_t at_roots = ((size_t)nroots + 1) * 8, at_cols = at_roots + nr * 4, bytes = at_cols + (size_t)total * 4;
+  PCUDA(grow_host(&P->h_in, &P->hcap_in, bytes));
   PCUDA(grow_host(&P->h_w, &P->hcap_w, (size_t)total));
-  PCUDA(grow_host(&P->h_roots, &P->hcap_roots, nr));
-  PCUDA(grow_dev(&P->d_loff, &P->cap_loff, (size_t)nroots + 1));
-  PCUDA(grow_dev(&P->d_lcols, &P->cap_lcols, (size_t)total));
+  PCUDA(grow_dev(&P->d_in, &P->cap_in, bytes));
   PCUDA(grow_dev(&P->d_w, &P->cap_w, (size_t)total));
-  PCUDA(grow_dev(&P->d_roots, &P->cap_roots, nr));
   PCUDA(grow_dev(&P->d_work, &P->cap_work, kPeelWorkHeader + 2 * kRegistryWords + nr));
   if (!grp[0].empty() && !P->d_slab) {
     P->slab_ctas = ctx_sms(c);
     P->slab_words = (uint64_t)kTierLMax * ((kTierLMax + 31) / 32);
     PCUDA(cudaMalloc((void **)&P->d_slab, P->slab_words * P->slab_ctas * sizeof(uint32_t)));
   }
-  memcpy(P->h_loff, loff, ((size_t)nroots + 1) * 8);
-  memcpy(P->h_lcols, lcols, (size_t)total * 4);
+  memcpy(P->h_in, loff, at_roots);
   size_t at = 0;
   for (auto &v : grp) {
-    memcpy(P->h_roots + at, v.data(), v.size() * 4);
+    if (!v.empty()) memcpy(P->h_in + at_roots + at * 4, v.data(), v.size() * 4);
     at += v.size();
   }
-  PCUDA(cudaMemcpyAsync(P->d_loff, P->h_loff, ((size_t)nroots + 1) * 8, cudaMemcpyHostToDevice, st));
-  PCUDA(cudaMemcpyAsync(P->d_lcols, P->h_lcols, (size_t)total * 4, cudaMemcpyHostToDevice, st));
-  PCUDA(cudaMemcpyAsync(P->d_roots, P->h_roots, nr * 4, cudaMemcpyHostToDevice, st));
+  memcpy(P->h_in + at_cols, lcols, (size_t)total * 4);
+  PCUDA(cudaMemcpyAsync(P->d_in, P->h_in, bytes, cudaMemcpyHostToDevice, st));
+  const uint32_t *const d_roots = reinterpret_cast<const uint32_t *>(P->d_in + at_roots);
   PCUDA(cudaMemsetAsync(P->d_work, 0, (kPeelWorkHeader + 2 * kRegistryWords + nr) * sizeof(uint32_t), st));
   uint32_t *const d_task = P->d_work + kPeelWorkHeader + 2 * kRegistryWords;
   dev::PassArgs a{};
@@ -156,8 +147,8 @@ kclpp_status peel_recount_run(PeelRecount *P, uint32_t nroots, const uint64_t *l
   a.bit_rows = graph_dev_bit_rows(P->g);
   a.bits = graph_dev_bits(P->g);
   a.err = ctx_err_word(c);
-  a.list_off = P->d_loff;
-  a.list_cols = P->d_lcols;
+  a.list_off = reinterpret_cast<const uint64_t *>(P->d_in);
+  a.list_cols = reinterpret_cast<const uint32_t *>(P->d_in + at_cols);
   a.pair_out = P->d_w;
   a.slab = P->d_slab;
   a.slab_words = P->slab_words;
@@ -168,7 +159,7 @@ kclpp_status peel_recount_run(PeelRecount *P, uint32_t nroots, const uint64_t *l
     if (v.empty()) continue;
     TierLaunch tl{};
     tl.tier = t == 0 ? 2 : (t == 1 ? 1 : 0);
-    tl.roots = P->d_roots + at;
+    tl.roots = d_roots + at;
     tl.num_roots = (uint32_t)v.size();
     tl.dmax = (uint32_t)(loff[v.front() + 1] - loff[v.front()]);
     tl.work = P->d_work + t;

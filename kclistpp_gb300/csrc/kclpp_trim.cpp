@@ -374,11 +374,12 @@ kclpp_status kclpp_trim(kclpp_ctx *ctx, const kclpp_edge_list *el, int kmax, int
     // reference does.  EXACT predicts the heap's next B pops (what it would
     // pop if no degree changed), recounts all of them at once on the GPU with
     // each one's live set as it would be at its pop, then commits pops while
-    // the heap's actual minimum is the predicted vertex: a committed pop's
-    // live set is then exactly the predicted one, so its counts are exact.
-    // The first pop that differs ends the batch; its count is recomputed in
-    // the next one.  B doubles while whole batches commit and shrinks to
-    // what the last batch committed otherwise.
+    // the heap's actual minimum is one of them and its live neighbours are the
+    // predicted ones -- in the predicted order they are, and in another order
+    // as long as no neighbour of it changed places with it -- so that its
+    // counts are exact.  The first pop that is not ends the batch; its count is
+    // recomputed in the next one.  B doubles while whole batches commit and
+    // shrinks to twice what the last batch committed otherwise.
     const auto t_peel = std::chrono::steady_clock::now();
     PeelHeap h(n2);
     for (uint32_t i = 0; i < n2; ++i) h.push(i, R->nck[i]);
@@ -460,17 +461,37 @@ kclpp_status kclpp_trim(kclpp_ctx *ctx, const kclpp_edge_list *el, int kmax, int
         }
         st = peel_recount_run(P, want, loff.data(), lcols.data(), gpu.data(), W.data());
         if (st != KCLPP_OK) return st;
-        uint32_t j = 0;
-        for (; j < want && h.key[0] == pred[j]; ++j) {
+        uint32_t done = 0;
+        bool in_order = true;  // every pop so far was the predicted one
+        while (bk.i + 1 < n2 && done < want) {
+          const uint32_t u = h.key[0];
+          if (mark[u] != gen) break;  // not recounted
+          const uint32_t j = mpos[u];
+          const uint32_t *L = lcols.data() + loff[j];
+          const uint32_t na = (uint32_t)(loff[j + 1] - loff[j]);
+          in_order &= u == pred[done];
+          if (!in_order) {
+            // u's counts hold whatever the order was, as long as its live
+            // neighbours are the ones they were taken over.
+            uint32_t now = 0, same = 0;
+            for (uint64_t q = cu[u]; q < cu[u + 1]; ++q) {
+              if (!h.live(au[q])) continue;
+              while (same < na && L[same] < au[q]) ++same;
+              if (same == na || L[same] != au[q]) { now = UINT32_MAX; break; }
+              ++now;
+            }
+            if (now != na) break;
+          }
           uint64_t v;
-          const uint32_t u = h.pop(&v);
-          bk.commit(h, u, v, lcols.data() + loff[j], (uint32_t)(loff[j + 1] - loff[j]), W.data() + loff[j]);
+          h.pop(&v);
+          bk.commit(h, u, v, L, na, W.data() + loff[j]);
           PS.gpu_roots += gpu[j];
+          ++done;
         }
         PS.batches++;
         PS.predicted += want;
-        PS.committed += j;
-        B = j == want ? std::min(2 * B, kMaxBatch) : std::max<uint32_t>(1, 2 * j);
+        PS.committed += done;
+        B = done == want ? std::min(2 * B, kMaxBatch) : std::max<uint32_t>(1, 2 * done);
       }
     }
     bk.finish(h, alive);
