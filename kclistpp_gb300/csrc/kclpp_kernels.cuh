@@ -952,28 +952,27 @@ struct TinyStream {
         return c + __reduce_add_sync(KCL_FULL, fell);
       }
     }
-    for (M rem = mask_of(act); rem; rem &= rem - 1) {
-      const int u = first(rem);
-      const M V = P & of(crow, u);
-      const uint32_t vu = of(v, u);
-      const bool own = vu < c;  // strict: ties stay with the earlier argmin
-      const uint32_t c0 = own ? vu : c;
-      uint32_t c1 = c0;
+    // One chain after another, the u's of a slot at a time: those of the first
+    // slot have candidates in it alone, and 32-bit masks serve.
 #pragma unroll
-      for (int q = 0; q < S; ++q) {
-        const uint32_t vm = S == 1 ? (uint32_t)V : (uint32_t)(V >> (32 * q));
-        if (S == 1 || vm) {
-          const uint32_t m = word_fixed_point((vm >> lane) & 1u ? (int)(v[q] - c1) : -1, lt);
-          v[q] += ((vm & ~m) >> lane) & 1u;
-          c1 += (uint32_t)__popc(m);
+    for (int z = 0; z < S; ++z) {
+      for (uint32_t rem = __ballot_sync(KCL_FULL, act[z]); rem; rem &= rem - 1) {
+        const int b = __ffs((int)rem) - 1;
+        const uint32_t vu = __shfl_sync(KCL_FULL, v[z], b);
+        const bool own = vu < c;  // strict: ties stay with the earlier argmin
+        const uint32_t c0 = own ? vu : c;
+        uint32_t c1 = c0;
+#pragma unroll
+        for (int q = 0; q <= z; ++q) {
+          const uint32_t vm = __shfl_sync(KCL_FULL, (uint32_t)(crow[z] >> (32 * q)), b) & (uint32_t)(P >> (32 * q));
+          if (z == 0 || vm) {
+            const uint32_t m = word_fixed_point((vm >> lane) & 1u ? (int)(v[q] - c1) : -1, lt);
+            v[q] += ((vm & ~m) >> lane) & 1u;
+            c1 += (uint32_t)__popc(m);
+          }
         }
-      }
-      if (own) {
-#pragma unroll
-        for (int q = 0; q < S; ++q)
-          if (32 * q + lane == u) v[q] += c1 - c0;
-      } else {
-        c = c1;
+        if (!own) c = c1;
+        else if (lane == b) v[z] += c1 - c0;
       }
     }
     return c;
