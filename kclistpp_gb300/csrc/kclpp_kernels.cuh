@@ -535,11 +535,12 @@ __device__ __forceinline__ uint32_t edges_in(const Bits<1> &P, const uint32_t *r
 // Triangles of G_s inside P, each once, as per-lane partial sums (the k = 5
 // count): a lane per member y of P walks the members z of P ∩ row(y) (below y
 // with BELOW) and adds |P ∩ row(y) ∩ row(z)| over the words those rows can
-// occupy.  scratch as in edges_in.
+// occupy.  scratch: cbuf_words(5, .) words.
 template <bool BELOW>
 __device__ __forceinline__ uint32_t triangles_in(const Bits<1> &P, const uint32_t *rows, int W, int lane,
                                                  uint32_t *scratch) {
-  uint16_t *members = reinterpret_cast<uint16_t *>(scratch + 32);
+  constexpr int cbuf_rows_at = 32;  // 64 rows of 64 bits, then the members
+  uint16_t *members = reinterpret_cast<uint16_t *>(scratch + 32 + 128);
   if (lane < W) scratch[lane] = P.w[0];
   const uint32_t lt = lanemask_lt();
   uint32_t total = 0;
@@ -553,6 +554,36 @@ __device__ __forceinline__ uint32_t triangles_in(const Bits<1> &P, const uint32_
   }
   __syncwarp();
   uint32_t c = 0;
+  if (total <= 64) {
+    // The rows among the members, as 64-bit masks: a step down the clique is
+    // then one word, where the rows as they stand are walked over all words
+    // they can occupy (a k = 5 Sim pass over RMAT-15 with planted communities,
+    // members mostly 20..50: 725 -> 658 us).
+    unsigned long long *R = reinterpret_cast<unsigned long long *>(scratch + cbuf_rows_at);
+    const uint32_t m0 = lane < total ? members[lane] : 0u, m1 = lane + 32 < total ? members[lane + 32] : 0u;
+    const uint32_t *col0 = rows + (m0 >> 5), *col1 = rows + (m1 >> 5);
+    const uint32_t bit0 = lane < total ? 1u << (m0 & 31) : 0u, bit1 = lane + 32 < total ? 1u << (m1 & 31) : 0u;
+    unsigned long long mine[2] = {0, 0};
+    for (uint32_t g = 0; g < total; ++g) {
+      const uint32_t o = (uint32_t)members[g] * (uint32_t)W;
+      const uint32_t b0 = __ballot_sync(KCL_FULL, (col0[o] & bit0) != 0);
+      const uint32_t b1 = total > 32 ? __ballot_sync(KCL_FULL, (col1[o] & bit1) != 0) : 0u;
+      const unsigned long long row = ((unsigned long long)b1 << 32 | b0) & (BELOW ? (1ull << g) - 1ull : ~0ull);
+      if (lane == (int)(g & 31u)) {
+        if (g < 32) mine[0] = row;
+        else mine[1] = row;
+        R[g] = row;
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const unsigned long long r = mine[q];
+      for (unsigned long long it = r; it; it &= it - 1) c += (uint32_t)__popcll(r & R[__ffsll((long long)it) - 1]);
+    }
+    __syncwarp();  // the next row reuses the scratch
+    return c;
+  }
   for (uint32_t i = lane; i < total; i += 32) {
     const int y = members[i];
     const uint32_t *ry = rows + (size_t)y * W;
@@ -598,9 +629,11 @@ __host__ __device__ inline size_t seq_warp_words(int k, uint32_t dmax, bool rows
 struct LayoutM {
   size_t list, tab, rows, base, acc, rel, rank, inv, dl, cbuf, total;
 };
-// Per-warp scratch of the k = 4 counting path (edges_in): P's words and its
-// members, compacted.
-__host__ __device__ inline size_t cbuf_words(uint32_t dmax) { return 32 + (dmax + 1) / 2; }
+// Per-warp scratch of the k = 4, 5 counting paths: P's words, (k = 5) the rows
+// among 64 members, and P's members, compacted.
+__host__ __device__ inline size_t cbuf_words(int k, uint32_t dmax) {
+  return (32 + (k == 5 ? 128 : 0) + ((size_t)dmax + 1) / 2 + 3) / 4 * 4;
+}
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 __host__ __device__ inline LayoutM layout_m(int mode, int k, uint32_t dmax, int nw, bool rows_in_smem) {
   LayoutM L;
@@ -617,7 +650,7 @@ __host__ __device__ inline LayoutM layout_m(int mode, int k, uint32_t dmax, int 
   L.rel = at; if (mode == MODE_SEQ && rows_in_smem) at = align16(at + (size_t)(dmax + 1) * 4);
   L.dl = at; if (mode == MODE_SEQ) at = align16(at + (size_t)nw * seq_warp_words(k, dmax, rows_in_smem) * 4);
   L.cbuf = at;
-  if (mode != MODE_SEQ && (k == 4 || k == 5) && rows_in_smem) at = align16(at + (size_t)nw * cbuf_words(dmax) * 4);
+  if (mode != MODE_SEQ && (k == 4 || k == 5) && rows_in_smem) at = align16(at + (size_t)nw * cbuf_words(k, dmax) * 4);
   L.total = at;
   return L;
 }
@@ -1913,7 +1946,7 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
   uint32_t *dl = reinterpret_cast<uint32_t *>(smem_raw + lay.dl) + (size_t)wid * seq_warp_words(K, a.dmax, ROWS_IN_SMEM);
   uint32_t *pair = K == 4 ? dl : dl + ((size_t)dmax + 4) / 4 * 4;
   uint32_t *rel = reinterpret_cast<uint32_t *>(smem_raw + lay.rel);
-  uint32_t *cbuf = reinterpret_cast<uint32_t *>(smem_raw + lay.cbuf) + (size_t)wid * cbuf_words(a.dmax);
+  uint32_t *cbuf = reinterpret_cast<uint32_t *>(smem_raw + lay.cbuf) + (size_t)wid * cbuf_words(K, a.dmax);
 
   __shared__ uint32_t s_idx, s_best[32], s_who[32];
   __shared__ int s_tau;
@@ -2028,13 +2061,22 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
     if constexpr (MODE == MODE_ORDER) {
       const unsigned long long ks = base[d];
       int t = 0;
-      for (int i = tid; i < d; i += NW * 32) {
-        const unsigned long long ki = base[i];
+      for (int i0 = wid * 32; i0 < d; i0 += NW * 32) {
+        // keys at or below i's before it, below i's after it: one comparison
+        // each but among the warp's own 32
+        const int i = i0 + lane;
+        const unsigned long long ki = i < d ? base[i] : 0ull;
+        const int mid = i0 + 32 < d ? i0 + 32 : d;
         int r = 0;
-        for (int j = 0; j < d; ++j) {
+#pragma unroll 4
+        for (int j = 0; j < i0; ++j) r += base[j] <= ki;
+        for (int j = i0; j < mid; ++j) {
           const unsigned long long kj = base[j];
           r += (kj < ki) || (kj == ki && j < i);
         }
+#pragma unroll 4
+        for (int j = mid; j < d; ++j) r += base[j] < ki;
+        if (i >= d) continue;
         rank[i] = (uint16_t)r;
         inv[r] = (uint16_t)i;
         t += (ki <= ks);
@@ -2093,6 +2135,12 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
       }
     } else {
       const int tau = (MODE == MODE_ORDER) ? s_tau : 0;
+      // COUNT, s's own share: the (k-1)-cliques of G_s.  A CTA that has the root
+      // to itself divides the rows' total by k - 1; CTAs that split one sum the
+      // cliques whose largest member is p, i.e. the (k-2)-cliques among p's
+      // neighbours below it, a second walk.  Explicit lists take no share.
+      // (Without the second walk: k = 4 count of RMAT-18 2.2 -> 1.7 ms.)
+      const bool low = MODE == MODE_COUNT && a.active && !a.list_off;
       unsigned long long mine = 0;
       for (;;) {
         int p = 0;
@@ -2103,28 +2151,25 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
         uint64_t c = 0;
         uint64_t c_low = 0;
         if constexpr (K == 4 && WPL == 1 && ROWS_IN_SMEM) {
-          c = warp_sum((uint64_t)edges_in<MODE == MODE_COUNT>(P, rows, W, lane, cbuf));
-          if constexpr (MODE == MODE_COUNT)
-            c_low = warp_sum((uint64_t)edges_in<true>(band(P, below_mask<WPL>(p, lane)), rows, W, lane, cbuf));
+          c = __reduce_add_sync(KCL_FULL, edges_in<MODE == MODE_COUNT>(P, rows, W, lane, cbuf));
+          if (MODE == MODE_COUNT && low)
+            c_low = __reduce_add_sync(KCL_FULL, edges_in<true>(band(P, below_mask<WPL>(p, lane)), rows, W, lane, cbuf));
         } else if constexpr (K == 5 && WPL == 1 && ROWS_IN_SMEM) {
-          c = warp_sum((uint64_t)triangles_in<MODE == MODE_COUNT>(P, rows, W, lane, cbuf));
-          if constexpr (MODE == MODE_COUNT)
-            c_low = warp_sum((uint64_t)triangles_in<true>(band(P, below_mask<WPL>(p, lane)), rows, W, lane, cbuf));
+          // at most C(1023, 3) triangles: 32 bits
+          c = __reduce_add_sync(KCL_FULL, triangles_in<MODE == MODE_COUNT>(P, rows, W, lane, cbuf));
+          if (MODE == MODE_COUNT && low)
+            c_low =
+                __reduce_add_sync(KCL_FULL, triangles_in<true>(band(P, below_mask<WPL>(p, lane)), rows, W, lane, cbuf));
         } else {
           c = warp_sum(cnt_warp<K - 2, MODE == MODE_COUNT, WPL>(P, rows, W, lane));
-          if constexpr (MODE == MODE_COUNT) {
-            // s's own share: the (k-1)-cliques of G_s whose largest member is p,
-            // i.e. the (k-2)-cliques among p's neighbours below it.  Summing
-            // these (instead of dividing the row total by k-1) stays exact when
-            // several CTAs split one root.
+          if (MODE == MODE_COUNT && low)
             c_low = warp_sum(cnt_warp<K - 2, true, WPL>(band(P, below_mask<WPL>(p, lane)), rows, W, lane));
-          }
         }
         if (lane == 0) {
           if (MODE == MODE_COUNT) {
             if (a.list_off) a.pair_out[o + p] = (unsigned long long)c;
             else if (c) atomicAdd(&a.out[list[p]], (unsigned long long)c);
-            mine += c_low;
+            mine += low ? c_low : c;
           } else if (p < tau) {
             if (c) atomicAdd(&a.out[list[inv[p]]], (unsigned long long)c);
           } else {
@@ -2135,8 +2180,9 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
       if (lane == 0 && mine) shared_add(&s_sum, mine);
       __syncthreads();
       if (tid == 0 && s_sum && !(MODE == MODE_COUNT && a.list_off)) {
-        atomicAdd(&a.out[s], s_sum);
-        if constexpr (IDENT && MODE == MODE_COUNT) atomicAdd(a.total, s_sum);
+        const unsigned long long own = MODE == MODE_COUNT && !low ? s_sum / (unsigned long long)(K - 1) : s_sum;
+        atomicAdd(&a.out[s], own);
+        if constexpr (IDENT && MODE == MODE_COUNT) atomicAdd(a.total, own);
       }
     }
     if (tid == 0 && a.active) a.active[blockIdx.x] = 0;
