@@ -61,6 +61,7 @@ constexpr int kSampleThreads = 512;
 constexpr uint32_t kWarpRoots = 1024;  // out-degree bound of the warp-per-edge kernel
 // Out-degree bounds and CTA widths of its launch groups: small roots have few
 // edges to share out and little shared memory to hold, so many narrow CTAs.
+// (Bounds 128 and 48 with 1024 threads for the largest: no difference.)
 constexpr uint32_t kGroupDeg[3] = {256, 64, 0};
 constexpr int kGroupThreads[3] = {512, 256, 128};
 constexpr int kPassThreads = 256;
@@ -263,7 +264,7 @@ struct WarpWalk {
 };
 
 template <int K>
-__global__ void __launch_bounds__(kSampleThreads) k_sample_warps(SampleArgs a) {
+__global__ void __launch_bounds__(kGroupThreads[0]) k_sample_warps(SampleArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int nw = (int)(blockDim.x >> 5), tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const WarpLayout lay = warp_layout(a.dmax, nw);
@@ -877,7 +878,8 @@ kclpp_status kclpp_sampling_extract(kclpp_ctx *c, kclpp_sampling *s, uint32_t T,
     kclpp_edge_list *el = nullptr;
     kclpp_graph *sg = nullptr;
     kclpp_status st2 = kclpp_edge_list_create(pairs.data(), rep->sub_e, &el);
-    if (st2 == KCLPP_OK) st2 = kclpp_build_graph(c, el, &sg);
+    // size, core value and count are those of any degeneracy order
+    if (st2 == KCLPP_OK) st2 = kclpp_build_graph_mode(c, el, KCLPP_ORDER_FAST, &sg);
     if (st2 == KCLPP_OK) st2 = kclpp_count_cliques(c, sg, k, nullptr, &rep->sub_cliques);
     uint32_t sn = 0, score = 0;
     uint64_t sm = 0;
