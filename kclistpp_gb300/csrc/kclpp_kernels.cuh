@@ -34,6 +34,7 @@
 // unmodified set, because the child set of u is P ∩ N+(u) over all of P.
 #pragma once
 
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 #include <utility>
@@ -2335,6 +2336,11 @@ cudaError_t launch_tier(const TierLaunch &t, dev::PassArgs a, cudaStream_t st) {
     const size_t sm = layout_m(MODE, K, t.dmax, nw, true).total;
     e = prepare(fn, lc, nw * 32, sm, &per_sm);
     if (e != cudaSuccess) return e;
+    // Shared loads: every stream in flight is blind to the others, so more of
+    // them at once cost passes.  At k >= 5 the kernel would hold 32 warps an SM
+    // (92 to 101 passes to a certified gap on a planted RMAT-13, 0.13 s); 24
+    // take 81 to 83, in 0.125 s.
+    if (MODE == MODE_SEQ && K >= 5 && a.shared_loads) per_sm = std::min(per_sm, std::max(1, 24 / nw));
     fn<<<persistent_grid(per_sm, t, 1, t.active != nullptr), nw * 32, sm, st>>>(a);
     return cudaGetLastError();
   }
