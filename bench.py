@@ -918,8 +918,9 @@ def main() -> None:
                     "note": "bytes = reference-equivalent bytes: the reference's per-root-edge gathers "
                             "(MakeSubgraph, kCDensestNoAtom.c:86-113) over every root edge of the pass; this "
                             "implementation reads impl_bytes of them (one induction per root vertex) and the DAG "
-                            "stays in L2, so DRAM traffic (from the committed ncu summary) is far below; the "
-                            "pass is bound by instruction issue (see issue)",
+                            "stays in L2, so DRAM traffic (from the committed ncu summary) is far below and frac "
+                            "can exceed 1: it rates the work those bytes stand for, not traffic; the pass is bound "
+                            "by instruction issue (see issue)",
                     "step_achieved": bpp * len(modes) / (ms / 1000.0) / 1e9}
         roofline["step_frac"] = roofline["step_achieved"] / peak
         # What actually bounds the pass: the dense core is L2-resident and the

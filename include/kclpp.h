@@ -157,7 +157,7 @@ kclpp_status kclpp_count_edges(kclpp_ctx *ctx, const kclpp_graph *g, uint32_t nu
  * shared-memory footprint and more CTAs per SM), tier L (beyond, up to 2048).
  * Work stealing lets CTAs without a root of their own join the roots other
  * CTAs are working on.  Defaults: tier_s_max 64, tier_s_max_seq 16, splits
- * 256 / 512, Seq stealing on, counting stealing off, 4 waves, widths 0 (auto),
+ * 256 / 512, Seq stealing on (for roots worth it at the pass's k), counting stealing off, 4 waves, widths 0 (auto),
  * concurrent groups on. */
 typedef struct {
   uint32_t tier_s_max;      /* counting kernels (k-clique degrees, Sim, PAVA): tier S bound, <= 64 */
@@ -170,7 +170,8 @@ typedef struct {
   uint32_t seq_warps[4];    /* Seq kernel, warps per CTA of the M1 (<= seq_split1), M2 (<= split2), */
                             /* M3 (<= 1024) and L root groups: 2, 4, 8, 12, 16, 20 or 24 (2 and 4:  */
                             /* many small CTAs, for groups of small roots); 0 = the width of 8..24 */
-                            /* that keeps the most warps resident per SM                           */
+                            /* that keeps the most warps resident per SM.  The widest: 24 at k <= 4, */
+                            /* 16 at k = 5, 6, 12 beyond (a larger request means that)              */
   int concurrent_tiers;     /* Seq kernel: launch a pass's root groups on forked streams (def. 1)  */
   uint32_t count_warps[4];  /* the counting / Sim kernels' widths of the same four groups:         */
                             /* 8, 16, 24 or 32; 0 = the most resident warps per SM                 */
