@@ -544,12 +544,16 @@ static kclpp_status run_tiers(kclpp_ctx *c, kclpp_graph *g, int mode, int k, dev
                               const Exec *ex = nullptr, int wave = -1) {
   const int sch = mode == dev::MODE_SEQ ? 1 : 0;
   const bool wv = mode == dev::MODE_SEQ && wave >= 0;
-  const std::vector<TierInfo> tiers = launch_plan(wv ? g->wave_tiers[wave] : g->tiers[sch], mode, k);
+  // Shared loads keep the schedule's groups and join any root: a stream there
+  // sees what others gave only when it starts, so lanes that run 32 streams at
+  // once, or CTAs that idle, cost passes to a certificate.
+  const std::vector<TierInfo> &groups = wv ? g->wave_tiers[wave] : g->tiers[sch];
+  const std::vector<TierInfo> tiers = a.shared_loads ? groups : launch_plan(groups, mode, k);
   const uint32_t base = wv ? g->wave_base[wave] : g->sched_base[sch];
   const Exec E = ex ? *ex : Exec{c->stream, g->d_work};
   // Work stealing pays off for the Seq chains (long, uneven root edges); the
   // counting kernels finish their roots quickly and by default do not steal.
-  const uint32_t steal_min = steal_from(mode, k);
+  const uint32_t steal_min = a.shared_loads ? 0u : steal_from(mode, k);
   bool steal = false;
   for (const TierInfo &t : tiers)
     steal |= t.tier > 0 && t.dmax >= steal_min && (mode == dev::MODE_SEQ ? g->sp.steal_seq : g->sp.steal_count) != 0;

@@ -1982,7 +1982,7 @@ __global__ void __launch_bounds__(warps_m<MODE, K>() * 32, min_ctas_m<MODE, K>()
     }
     if (stealing) {
       if (!a.active) break;
-      const uint32_t least = ((uint32_t)NW * steal_quarters<MODE, K>() + 3u) / 4u;
+      const uint32_t least = a.shared_loads ? 2u : ((uint32_t)NW * steal_quarters<MODE, K>() + 3u) / 4u;
       idx = find_victim<IDENT>(a, K - 1, least > 2u ? least : 2u, s_best, s_who);
       if (idx == UINT32_MAX) break;
       if (tid == 0) atomicAdd(a.task_next + idx, 1u << kTaskBits);
@@ -2337,10 +2337,11 @@ cudaError_t launch_tier(const TierLaunch &t, dev::PassArgs a, cudaStream_t st) {
     e = prepare(fn, lc, nw * 32, sm, &per_sm);
     if (e != cudaSuccess) return e;
     // Shared loads: every stream in flight is blind to the others, so more of
-    // them at once cost passes.  At k >= 5 the kernel would hold 32 warps an SM
-    // (92 to 101 passes to a certified gap on a planted RMAT-13, 0.13 s); 24
-    // take 81 to 83, in 0.125 s.
-    if (MODE == MODE_SEQ && K >= 5 && a.shared_loads) per_sm = std::min(per_sm, std::max(1, 24 / nw));
+    // them at once cost passes.  24 warps an SM instead of what fits: a planted
+    // RMAT-13 at k = 5 takes 81 to 83 passes to a certified gap (92 to 101), a
+    // planted RMAT-12 at k = 3 is certified from 64 passes in 60 of 60 runs (58),
+    // and its pass takes 96 us (129).
+    if (MODE == MODE_SEQ && a.shared_loads) per_sm = std::min(per_sm, std::max(1, 24 / nw));
     fn<<<persistent_grid(per_sm, t, 1, t.active != nullptr), nw * 32, sm, st>>>(a);
     return cudaGetLastError();
   }
