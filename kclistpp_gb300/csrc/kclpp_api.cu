@@ -118,6 +118,7 @@ struct kclpp_graph {
   uint32_t *d_level = nullptr;
   uint32_t *d_work = nullptr;   // scheduler words (work_words)
   uint32_t num_roots = 0;
+  uint64_t schedule_gen = 0;    // builds of the schedule: recorded launches hold an older one's addresses
   size_t work_cap = 0;
   unsigned long long *d_scalar = nullptr;
   uint32_t *d_slab = nullptr;
@@ -298,6 +299,7 @@ static inline uint32_t wave_of(uint32_t s, uint32_t B) { return (uint32_t)(s * 2
 // that the longest CTAs start first.
 static kclpp_status build_schedule(kclpp_ctx *c, kclpp_graph *g) {
   const HostDag &D = g->dag;
+  ++g->schedule_gen;
   auto deg = [&](uint32_t s) { return (uint32_t)(D.off[s + 1] - D.off[s]); };
   auto by_work = [&](uint32_t a, uint32_t b) {
     const uint32_t da = deg(a), db = deg(b);
@@ -1356,7 +1358,7 @@ struct kclpp_batch {
   int exec_kernel = -1;
   std::vector<int> exec_ks;
   uint32_t exec_passes = 0;
-  kclpp_schedule exec_sched{};  // the union graph's schedule when the graph was captured
+  uint64_t exec_gen = 0;  // the union graph's schedule_gen when the graph was captured
 };
 
 static void batch_release(kclpp_batch *b) {
@@ -1480,13 +1482,15 @@ kclpp_status kclpp_batch_run(kclpp_ctx *c, kclpp_batch *b, int kernel, const int
   for (int i = 0; i < nk; ++i) KCL_TRY(check_k(ks[i], kernel == KCLPP_KERNEL_SEQ ? 3 : 2));
   KCL_TRY(set_device(c));
   kclpp_graph *g = b->g;
+  KCL_TRY(check_unsharded(g, "kclpp_batch_run"));
   const uint32_t n = g->dag.n;
   if (!n) return KCLPP_OK;
   const std::vector<int> want(ks, ks + nk);
-  // A schedule set on the union graph since the capture (kclpp_autotune,
-  // kclpp_graph_set_schedule) changes the launches: capture again.
+  // A schedule built on the union graph since the capture (kclpp_autotune,
+  // kclpp_graph_set_schedule, kclpp_graph_shard) has freed the root array that
+  // the captured launches read, even where it is the same schedule again.
   const bool same = b->exec && b->exec_kernel == kernel && b->exec_ks == want && b->exec_passes == passes &&
-                    memcmp(&b->exec_sched, &g->sp, sizeof g->sp) == 0;
+                    b->exec_gen == g->schedule_gen;
   if (!same) {
     batch_release(b);
     if (!b->fork) KCL_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
@@ -1516,7 +1520,7 @@ kclpp_status kclpp_batch_run(kclpp_ctx *c, kclpp_batch *b, int kernel, const int
     b->exec_kernel = kernel;
     b->exec_ks = want;
     b->exec_passes = passes;
-    b->exec_sched = g->sp;
+    b->exec_gen = g->schedule_gen;
   }
   KCL_CUDA(cudaGraphLaunch(b->exec, c->stream));
   c->launches++;
