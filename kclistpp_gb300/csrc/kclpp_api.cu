@@ -486,11 +486,12 @@ static void free_graph_dev(kclpp_graph *g) {
   cudaFree(g->d_work); cudaFree(g->d_scalar); cudaFree(g->d_slab);
 }
 
-// Where a pass runs: its stream and its scheduler counters.  Concurrent passes
-// (the batch's k values) each need their own counters.
+// Where a pass runs: its stream, its scheduler counters and tier L's rows.
+// Concurrent passes (the batch's k values) each need their own.
 struct Exec {
   cudaStream_t st;
   uint32_t *work;  // work_words(roots, kMaxGroups)
+  uint32_t *slab;  // slab_words * slab_ctas words, or nullptr: no root in tier L
 };
 
 // The launches of one pass at clique size k, from the schedule's groups.
@@ -552,7 +553,7 @@ static kclpp_status run_tiers(kclpp_ctx *c, kclpp_graph *g, int mode, int k, dev
   const std::vector<TierInfo> &groups = wv ? g->wave_tiers[wave] : g->tiers[sch];
   const std::vector<TierInfo> tiers = a.shared_loads ? groups : launch_plan(groups, mode, k);
   const uint32_t base = wv ? g->wave_base[wave] : g->sched_base[sch];
-  const Exec E = ex ? *ex : Exec{c->stream, g->d_work};
+  const Exec E = ex ? *ex : Exec{c->stream, g->d_work, g->d_slab};
   // Work stealing pays off for the Seq chains (long, uneven root edges); the
   // counting kernels finish their roots quickly and by default do not steal.
   const uint32_t steal_min = a.shared_loads ? 0u : steal_from(mode, k);
@@ -577,7 +578,7 @@ static kclpp_status run_tiers(kclpp_ctx *c, kclpp_graph *g, int mode, int k, dev
   a.off = g->d_off;
   a.cols = g->d_cols;
   a.err = c->d_err;
-  a.slab = g->d_slab;
+  a.slab = E.slab;
   a.slab_words = g->slab_words;
   a.bit_rows = g->d_bit_rows;
   a.bits = g->d_bits;
@@ -1344,6 +1345,7 @@ struct BatchBranch {
   cudaStream_t st = nullptr;
   cudaEvent_t join = nullptr;
   uint32_t *work = nullptr;
+  uint32_t *slab = nullptr;  // tier L's rows (the branches run side by side)
   unsigned long long *buf[2] = {nullptr, nullptr};  // Seq ping-pong, or Sim counts in buf[0]
   double *rho = nullptr;
   void *result = nullptr;  // device vector holding the branch's final r / rho
@@ -1365,7 +1367,7 @@ static void batch_release(kclpp_batch *b) {
   for (auto &x : b->br) {
     if (x.st) cudaStreamDestroy(x.st);
     if (x.join) cudaEventDestroy(x.join);
-    cudaFree(x.work); cudaFree(x.buf[0]); cudaFree(x.buf[1]); cudaFree(x.rho);
+    cudaFree(x.work); cudaFree(x.slab); cudaFree(x.buf[0]); cudaFree(x.buf[1]); cudaFree(x.rho);
   }
   b->br.clear();
   if (b->exec) cudaGraphExecDestroy(b->exec);
@@ -1442,7 +1444,7 @@ static kclpp_status batch_record(kclpp_ctx *c, kclpp_batch *b, int kernel, uint3
   KCL_CUDA(cudaEventRecord(b->fork, c->stream));
   for (auto &x : b->br) {
     KCL_CUDA(cudaStreamWaitEvent(x.st, b->fork, 0));
-    const Exec E{x.st, x.work};
+    const Exec E{x.st, x.work, x.slab};
     if (kernel == KCLPP_KERNEL_SEQ) {
       KCL_CUDA(cudaMemsetAsync(x.buf[0], 0, (size_t)n * 8, x.st));
       int cur = 0;
@@ -1501,6 +1503,7 @@ kclpp_status kclpp_batch_run(kclpp_ctx *c, kclpp_batch *b, int kernel, const int
       KCL_CUDA(cudaStreamCreateWithFlags(&x.st, cudaStreamNonBlocking));
       KCL_CUDA(cudaEventCreateWithFlags(&x.join, cudaEventDisableTiming));
       KCL_TRY(dalloc(&x.work, work_words(g->num_roots, kMaxGroups)));
+      if (g->d_slab) KCL_TRY(dalloc(&x.slab, g->slab_words * g->slab_ctas));
       KCL_TRY(dalloc(&x.buf[0], n));
       if (kernel == KCLPP_KERNEL_SEQ) KCL_TRY(dalloc(&x.buf[1], n));
       else KCL_TRY(dalloc(&x.rho, n));

@@ -10,6 +10,7 @@
  *                              that a launch takes on the clock that events read
  *   fake_launches(name)        launches of kernels whose name holds `name`
  *   fake_instantiations()      CUDA graphs instantiated
+ *   fake_allocations(n)        device allocations of at least n bytes, freed ones too
  */
 #include <stdio.h>
 #include <stdlib.h>
@@ -40,6 +41,13 @@ unsigned long fake_launches(const char *name) {
   for (int i = 0; i < nkernels; ++i)
     if (strstr(kernels[i].name, name)) n += kernels[i].launches;
   return n;
+}
+static size_t sizes[1 << 16];
+static unsigned nsizes;
+unsigned long fake_allocations(size_t n) {
+  unsigned long c = 0;
+  for (unsigned i = 0; i < nsizes; ++i) c += sizes[i] >= n;
+  return c;
 }
 unsigned long fake_instantiations(void) { return ninstantiations; }
 
@@ -138,6 +146,7 @@ cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t e) { return e == cudaErrorMemoryAllocation ? "out of memory" : "error"; }
 cudaError_t cudaMalloc(void **p, size_t n) {
   if (malloc_limit && n > malloc_limit) return cudaErrorMemoryAllocation;
+  if (nsizes < sizeof sizes / sizeof *sizes) sizes[nsizes++] = n;
   *p = calloc(1, n);
   return *p ? cudaSuccess : cudaErrorMemoryAllocation;
 }

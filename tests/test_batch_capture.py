@@ -1,4 +1,7 @@
-"""A batch replays the CUDA graph it captured only while the union graph's
+"""What a batch's concurrent branches hold of their own, and when its captured
+CUDA graph may be replayed.
+
+A batch replays the CUDA graph it captured only while the union graph's
 schedule is the very one it was captured with: building a schedule again, even
 an equal one, frees the root array that the captured launches read.
 
@@ -73,6 +76,44 @@ def test_equal_schedule_again_captures_again(ctx):
         for g in hold:
             g.close()
     assert min(launches) > 1  # one launch would be a replay
+    b.close()
+
+
+def _deep():
+    """Roots of out-degree 1100 (rows in global memory), few cliques: two halves
+    joined completely, a sparse graph inside each."""
+    a, rng = 1100, np.random.default_rng(4)
+    parts = [np.stack(np.meshgrid(np.arange(a), np.arange(a, 2 * a), indexing="ij"), -1).reshape(-1, 2)]
+    for base in (0, a):
+        i, j = np.triu_indices(a, 1)
+        keep = rng.random(len(i)) < 2.0 / a
+        parts.append(np.stack([base + i[keep], base + j[keep]], axis=1))
+    return K.EdgeList.from_pairs(np.concatenate(parts).astype(np.uint32))
+
+
+def test_each_branch_has_its_rows_in_global_memory(tmp_path):
+    fake_cuda.run(tmp_path, """
+        from tests.test_batch_capture import _deep
+        b = K.Batch(ctx, [_deep()])
+        slab = 152 * 2048 * 64 * 4
+        before = fake.fake_allocations(slab)
+        b.run(K.KERNEL_SEQ, [3, 4, 5], 1)
+        assert fake.fake_allocations(slab) - before == 3
+        """)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kernel", [K.KERNEL_SEQ, K.KERNEL_ORDER])
+def test_branches_over_deep_roots_equal_single_runs(ctx, kernel):
+    el, ks = _deep(), [3, 4, 5]
+    b = K.Batch(ctx, [el, K.chung_lu(2000, 12.0, 2.4, seed=63)])
+    g = K.build_graph(ctx, el)
+    assert g.core > 1024
+    for _ in range(3):
+        out = b.run(kernel, ks, 2)
+        for ki, k in enumerate(ks):
+            want = K.seq_passes(g, k, 2) if kernel == K.KERNEL_SEQ else K.sim_passes(g, k, 2)
+            assert np.array_equal(out[ki, b.slice(0)].view(np.uint64), want.view(np.uint64)), k
     b.close()
 
 
