@@ -503,7 +503,11 @@ struct Exec {
 //  * Counting, k >= 5: warp-per-root roots above 32 members, whose rows a lane
 //    counts alone, go to a CTA: a core of out-degree 120 at k = 5, 424 us a Sim
 //    pass with the warp, 228 with the CTA; at k = 4 there is no difference.
-static std::vector<TierInfo> launch_plan(const std::vector<TierInfo> &tiers, int mode, int k) {
+// Both are what a tier S bound left at its default means; a program that sets
+// another bound has exactly that one, at every k.
+static std::vector<TierInfo> launch_plan(const std::vector<TierInfo> &tiers, const kclpp_schedule &sp, int mode,
+                                         int k) {
+  if (mode == dev::MODE_SEQ ? sp.tier_s_max_seq != kTierSMaxSeq : sp.tier_s_max != kTierSMax) return tiers;
   std::vector<TierInfo> plan;
   for (TierInfo t : tiers) {
     const TierInfo *prev = plan.empty() ? nullptr : &plan.back();
@@ -551,7 +555,7 @@ static kclpp_status run_tiers(kclpp_ctx *c, kclpp_graph *g, int mode, int k, dev
   // sees what others gave only when it starts, so lanes that run 32 streams at
   // once, or CTAs that idle, cost passes to a certificate.
   const std::vector<TierInfo> &groups = wv ? g->wave_tiers[wave] : g->tiers[sch];
-  const std::vector<TierInfo> tiers = a.shared_loads ? groups : launch_plan(groups, mode, k);
+  const std::vector<TierInfo> tiers = a.shared_loads ? groups : launch_plan(groups, g->sp, mode, k);
   const uint32_t base = wv ? g->wave_base[wave] : g->sched_base[sch];
   const Exec E = ex ? *ex : Exec{c->stream, g->d_work, g->d_slab};
   // Work stealing pays off for the Seq chains (long, uneven root edges); the
