@@ -41,6 +41,7 @@ struct PendingTime {
   int mode, tier;
   uint32_t dmax;
   cudaEvent_t a, b;
+  int bucket;  // the root group whose width the launch took, or -1
 };
 
 struct kclpp_ctx {
@@ -612,7 +613,7 @@ static kclpp_status run_tiers(kclpp_ctx *c, kclpp_graph *g, int mode, int k, dev
     tl.max_grid = t.tier == 2 ? g->slab_ctas : 0;
     tl.warps = t.bucket < 0 ? 0 : (int)(mode == dev::MODE_SEQ ? g->sp.seq_warps[t.bucket] : g->sp.count_warps[t.bucket]);
     cudaError_t e = cudaSuccess;
-    PendingTime pt{mode, t.tier, t.dmax, nullptr, nullptr};
+    PendingTime pt{mode, t.tier, t.dmax, nullptr, nullptr, t.bucket};
     const bool prof = c->profile && !ex;
     if (prof) {
       pt.a = take_event(c);
@@ -1201,9 +1202,11 @@ static kclpp_status time_pass(kclpp_ctx *c, kclpp_graph *g, int k, int mode, flo
   return check_err(c);
 }
 
-// Per-launch times of one pass of `mode` (after a warm-up pass), in launch
-// order: the per-launch events of the profiler, kept apart from the caller's.
-static kclpp_status time_tiers(kclpp_ctx *c, kclpp_graph *g, int k, int mode, std::vector<float> &ms) {
+// Times of one pass of `mode` (after a warm-up pass) by root group, as the pass
+// launched them (launch_plan): ms[b] is the sum over the launches whose width is
+// group b's, or below 0 where none was.  The events are the profiler's, kept
+// apart from the caller's.
+static kclpp_status time_tiers(kclpp_ctx *c, kclpp_graph *g, int k, int mode, float (&ms)[4]) {
   const size_t bytes = (size_t)g->dag.n * 8;
   std::vector<PendingTime> saved;
   saved.swap(c->pending);
@@ -1225,11 +1228,11 @@ static kclpp_status time_tiers(kclpp_ctx *c, kclpp_graph *g, int k, int mode, st
   }
   c->profile = was;
   if (st == KCLPP_OK && cudaStreamSynchronize(c->stream) != cudaSuccess) st = set_error(KCLPP_ERR_CUDA, "sync failed");
-  ms.clear();
+  for (float &t : ms) t = -1.f;
   for (auto &p : c->pending) {
     float t = 0.f;
     if (st == KCLPP_OK) cudaEventElapsedTime(&t, p.a, p.b);
-    ms.push_back(t);
+    if (p.bucket >= 0) ms[p.bucket] = std::max(ms[p.bucket], 0.f) + t;
     c->event_pool.push_back(p.a);
     c->event_pool.push_back(p.b);
   }
@@ -1290,7 +1293,8 @@ kclpp_status kclpp_autotune(kclpp_ctx *c, kclpp_graph *g, int k, int kernel, kcl
   }
   {
     // Warps per CTA, chosen per root group: the groups run as separate
-    // launches, so each one's width is tuned on its own launch time.
+    // launches, so each one's width is tuned on its own launches' time.  A group
+    // without a launch of its own at this k keeps the width it had.
     const bool sq = mode == dev::MODE_SEQ;
     const uint32_t seq_w[7] = {2, 4, 8, 12, 16, 20, 24}, cnt_w[4] = {8, 16, 24, 32};
     const uint32_t *widths = sq ? seq_w : cnt_w;
@@ -1304,17 +1308,14 @@ kclpp_status kclpp_autotune(kclpp_ctx *c, kclpp_graph *g, int k, int kernel, kcl
       (sq ? x.concurrent_tiers : x.concurrent_count) = 0;  // each group's own launch time
       for (int b = 0; b < 4; ++b) (sq ? x.seq_warps : x.count_warps)[b] = w;
       KCL_TRY(kclpp_graph_set_schedule(c, g, &x));
-      std::vector<float> ms;
+      float ms[4];
       KCL_TRY(time_tiers(c, g, k, mode, ms));
-      const std::vector<TierInfo> &tiers = g->tiers[sq ? 1 : 0];
-      for (size_t i = 0; i < tiers.size() && i < ms.size(); ++i) {
-        const int b = tiers[i].bucket;
-        if (b >= 0 && ms[i] < bt[b]) {
-          bt[b] = ms[i];
+      for (int b = 0; b < 4; ++b)
+        if (ms[b] >= 0.f && ms[b] < bt[b]) {
+          bt[b] = ms[b];
           (sq ? tuned.seq_warps : tuned.count_warps)[b] = w;
           any = true;
         }
-      }
     }
     if (any) {
       KCL_TRY(kclpp_graph_set_schedule(c, g, &tuned));

@@ -16,7 +16,7 @@ import kclistpp_gb300 as K
 fake = C.CDLL(None)
 fake.fake_launches.restype = fake.fake_instantiations.restype = fake.fake_allocations.restype = C.c_ulong
 fake.fake_malloc_limit.argtypes = fake.fake_allocations.argtypes = [C.c_size_t]
-COST = C.CFUNCTYPE(C.c_double, C.c_char_p, C.c_uint, C.c_ulong)
+COST = C.CFUNCTYPE(C.c_double, C.c_char_p, C.c_uint, C.c_uint, C.c_ulong)
 ctx = K.Context(0)
 """
 

@@ -6,7 +6,7 @@
  * A test steers it through the fake_* functions:
  *   fake_malloc_limit(n)       device allocations above n bytes fail (0: none do)
  *   fake_status_word(v)        from now on every 4-byte read from the device gives v
- *   fake_cost(f)               f(kernel name, threads per block, launches so far): ms
+ *   fake_cost(f)               f(kernel name, blocks, threads per block, launches so far): ms
  *                              that a launch takes on the clock that events read
  *   fake_launches(name)        launches of kernels whose name holds `name`
  *   fake_instantiations()      CUDA graphs instantiated
@@ -30,12 +30,12 @@ static int have_status;
 static unsigned status_word;
 static unsigned long nlaunches, ninstantiations;
 static double now_ms;
-static double (*cost_fn)(const char *, unsigned, unsigned long);
+static double (*cost_fn)(const char *, unsigned, unsigned, unsigned long);
 
 void fake_malloc_limit(size_t n) { malloc_limit = n; }
 void fake_status_word(unsigned v) { have_status = 1; status_word = v; }
 void fake_status_clear(void) { have_status = 0; }
-void fake_cost(double (*f)(const char *, unsigned, unsigned long)) { cost_fn = f; }
+void fake_cost(double (*f)(const char *, unsigned, unsigned, unsigned long)) { cost_fn = f; }
 unsigned long fake_launches(const char *name) {
   unsigned long n = 0;
   for (int i = 0; i < nkernels; ++i)
@@ -110,11 +110,11 @@ cudaError_t __cudaGetKernel(cudaKernel_t *k, const void *fn) {
   return cudaSuccess;
 }
 cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 grid, dim3 block, void **args, size_t smem, cudaStream_t st) {
-  (void)grid; (void)args; (void)smem; (void)st;
+  (void)args; (void)smem; (void)st;
   for (int i = 0; i < nkernels; ++i)
     if (kernels[i].fn == (const void *)k) {
       kernels[i].launches++;
-      now_ms += cost_fn ? cost_fn(kernels[i].name, block.x, nlaunches) : 1.0;
+      now_ms += cost_fn ? cost_fn(kernels[i].name, grid.x, block.x, nlaunches) : 1.0;
       nlaunches++;
       return cudaSuccess;
     }
