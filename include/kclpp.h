@@ -230,7 +230,9 @@ void kclpp_batch_free(kclpp_batch *b);
 
 /* ---- k-clique counts (A16 on the DAG) ----------------------------------- */
 /* Number of k-cliques and, if per_vertex != NULL, the k-clique degree of every
- * vertex (onepass/recursion, kClistCoreTrim.c:368-416). */
+ * vertex (onepass/recursion, kClistCoreTrim.c:368-416).  Here and in the Seq and
+ * Sim calls below, a call that fails leaves the caller's host vectors as they
+ * were. */
 kclpp_status kclpp_count_cliques(kclpp_ctx *ctx, const kclpp_graph *g, int k,
                                  uint64_t *per_vertex, uint64_t *total);
 /* The same k-clique degrees for callers that cannot allocate device memory

@@ -208,8 +208,9 @@ static kclpp_status check_err(kclpp_ctx *c) {
 // Copies of a call that takes and returns host vectors, through the context's
 // pinned megabyte where they fit: a copy to or from pageable memory waits in the
 // driver, two or three times a call (the triangle counts of 10,000 vertices: 59
-// us with direct copies, 54 staged).  Larger vectors are copied directly.  finish() ends the call: it
-// reads the status word, waits, and hands the results over.
+// us with direct copies, 54 staged).  Larger vectors are copied directly.
+// finish() ends the call: it reads the status word, waits, and hands the results
+// over, so that a call that fails leaves the caller's vectors as they were.
 class Staged {
  public:
   explicit Staged(kclpp_ctx *c) : c_(c) { c->pin_used = 0; }
@@ -228,16 +229,23 @@ class Staged {
     return KCLPP_OK;
   }
   kclpp_status down(void *host, const void *dev, size_t bytes) {
-    if (unsigned char *p = room(bytes)) {
-      out_.push_back({host, p, bytes});
-      host = p;
-    }
-    KCL_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, c_->stream));
+    unsigned char *p = room(bytes);
+    out_.push_back({host, p ? p : dev, bytes, p != nullptr});
+    if (p) KCL_CUDA(cudaMemcpyAsync(p, dev, bytes, cudaMemcpyDeviceToHost, c_->stream));
     return KCLPP_OK;
   }
   kclpp_status finish() {
     KCL_TRY(check_err(c_));
-    for (const Out &o : out_) memcpy(o.host, o.pinned, o.bytes);
+    bool direct = false;
+    for (const Out &o : out_) {
+      if (o.pinned) {
+        memcpy(o.host, o.from, o.bytes);
+      } else {
+        KCL_CUDA(cudaMemcpyAsync(o.host, o.from, o.bytes, cudaMemcpyDeviceToHost, c_->stream));
+        direct = true;
+      }
+    }
+    if (direct) KCL_CUDA(cudaStreamSynchronize(c_->stream));
     c_->pin_used = 0;
     return KCLPP_OK;
   }
@@ -245,8 +253,9 @@ class Staged {
  private:
   struct Out {
     void *host;
-    const unsigned char *pinned;
+    const void *from;  // the pinned copy, or the device's vector
     size_t bytes;
+    bool pinned;
   };
   unsigned char *room(size_t bytes) {
     const size_t at = (c_->pin_used + 15) & ~(size_t)15;
