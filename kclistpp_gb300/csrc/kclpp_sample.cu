@@ -83,6 +83,7 @@ struct SampleArgs {
   uint8_t *wave;
   unsigned long long cap;
   unsigned long long *count;
+  unsigned long long *wave_at;  // next free row of each wave, or nullptr: rows in any order, counted in count
   const uint4 *bit_rows;  // the graph's bitmap rows (dev::PassArgs)
   const uint32_t *bits;
 };
@@ -94,16 +95,17 @@ struct DevEmit {
   uint32_t *rows;
   uint8_t *wave;
   unsigned long long cap;
-  unsigned long long *count;
+  unsigned long long *count, *wave_at;
   uint64_t threshold;
   bool all;
   uint32_t waves;
   __device__ __forceinline__ void operator()(uint64_t h, const uint32_t *path, uint32_t v) const {
     if (!smp::kept(h, threshold, all)) return;
-    const unsigned long long pos = atomicAdd(count, 1ull);
+    const uint32_t w = smp::wave_of(h, waves);
+    const unsigned long long pos = atomicAdd(wave_at ? wave_at + w : count, 1ull);
     if (pos >= cap) return;  // counted only: the host grows the buffer and samples again
     smp::write_row<K>(rows + pos * K, list, s, path, v);
-    wave[pos] = (uint8_t)smp::wave_of(h, waves);
+    wave[pos] = (uint8_t)w;
   }
 };
 
@@ -135,7 +137,7 @@ __global__ void __launch_bounds__(kSampleThreads) k_sample(SampleArgs a) {
     for (uint32_t i = threadIdx.x; i < d; i += blockDim.x)
       smp::build_row(i, list, a.off, a.cols, rows + (size_t)i * a.ws);
     __syncthreads();
-    DevEmit<K> em{list, s, a.rows, a.wave, a.cap, a.count, a.threshold, a.all != 0, a.waves};
+    DevEmit<K> em{list, s, a.rows, a.wave, a.cap, a.count, a.wave_at, a.threshold, a.all != 0, a.waves};
     const uint64_t hs = smp::vertex_key(a.seed, s);
     for (;;) {
       const uint32_t t = atomicAdd(&s_edge, 1u);
@@ -180,11 +182,15 @@ struct WarpWalk {
   // A kept clique (path[0 .. K - 3], then u, v): appended by the lanes that are here.
   __device__ __forceinline__ void emit(uint64_t h, uint32_t u, uint32_t v) {
     if (!smp::kept(h, a.threshold, a.all != 0)) return;
-    const uint32_t here = __activemask();
-    const int first = __ffs((int)here) - 1;
     unsigned long long pos = 0;
-    if (lane == first) pos = atomicAdd(a.count, (unsigned long long)__popc(here));
-    pos = __shfl_sync(here, pos, first) + (uint32_t)__popc(here & dev::lanemask_lt());
+    if (a.wave_at) {
+      pos = atomicAdd(a.wave_at + smp::wave_of(h, a.waves), 1ull);
+    } else {
+      const uint32_t here = __activemask();
+      const int first = __ffs((int)here) - 1;
+      if (lane == first) pos = atomicAdd(a.count, (unsigned long long)__popc(here));
+      pos = __shfl_sync(here, pos, first) + (uint32_t)__popc(here & dev::lanemask_lt());
+    }
     if (pos >= a.cap) return;  // counted only: the host grows the buffer and samples again
     uint32_t *row = a.rows + pos * K;
     row[0] = list[v];
@@ -527,8 +533,11 @@ kclpp_status launch_k(int k, kclpp_ctx *c, kclpp_sampling *S, const SampleArgs &
   }
 }
 
-// The kept rows grouped by wave, in buffers of their number.
-kclpp_status group_by_wave(kclpp_ctx *c, kclpp_sampling *S) {
+// The kept rows grouped by wave, in buffers of their number.  Where the device
+// has no room for a second copy of them, they are drawn again in place:
+// redraw(at) samples with every row at the cursor of its wave.
+template <typename Redraw>
+kclpp_status group_by_wave(kclpp_ctx *c, kclpp_sampling *S, Redraw &&redraw) {
   S->wave_at.assign(smp::kMaxWaves + 1, 0);
   if (!S->sampled) return KCLPP_OK;
   cudaStream_t st = ctx_stream(c);
@@ -540,8 +549,10 @@ kclpp_status group_by_wave(kclpp_ctx *c, kclpp_sampling *S) {
   } t;
   const size_t words = smp::kMaxWaves + 1;
   SCUDA(dalloc(&t.cnt, words));
-  SCUDA(dalloc(&t.rows, (size_t)S->sampled * S->k));
-  SCUDA(dalloc(&t.wave, (size_t)S->sampled));
+  cudaError_t room = dalloc(&t.rows, (size_t)S->sampled * S->k);
+  if (room == cudaSuccess) room = dalloc(&t.wave, (size_t)S->sampled);
+  if (room == cudaErrorMemoryAllocation) cudaGetLastError();
+  else SCUDA(room);
   SCUDA(cudaMemsetAsync(t.cnt, 0, words * 8, st));
   const uint32_t grid = (uint32_t)std::min<uint64_t>((S->sampled + 2047) / 2048, (uint64_t)ctx_sms(c) * 8);
   k_wave_count<<<grid, 256, 0, st>>>(S->d_wave, S->sampled, t.cnt);
@@ -550,6 +561,12 @@ kclpp_status group_by_wave(kclpp_ctx *c, kclpp_sampling *S) {
   SCUDA(cudaStreamSynchronize(st));
   for (size_t w = 1; w < words; ++w) S->wave_at[w] += S->wave_at[w - 1];
   SCUDA(cudaMemcpyAsync(t.cnt, S->wave_at.data(), words * 8, cudaMemcpyHostToDevice, st));
+  if (room != cudaSuccess) {
+    ctx_count_launch(c, 1);
+    cudaFree(t.rows);  // the redraw may need a slab
+    t.rows = nullptr;
+    return redraw(t.cnt);
+  }
   k_wave_move<<<grid, 256, 0, st>>>(S->d_rows, S->d_wave, S->sampled, S->k, t.cnt, t.rows, t.wave);
   SCUDA(cudaGetLastError());
   SCUDA(cudaStreamSynchronize(st));
@@ -588,20 +605,10 @@ kclpp_status sample(kclpp_ctx *c, kclpp_sampling *S) {
     if (d_work) cudaFree(d_work);
     if (d_count) cudaFree(d_count);
   };
-  kclpp_status status = KCLPP_OK;
-  for (int attempt = 0; attempt < 2; ++attempt) {
-    cudaError_t e = cudaSuccess;
-    if (e == cudaSuccess && !d_work) e = dalloc(&d_work, 4);
-    if (e == cudaSuccess && !d_count) e = dalloc(&d_count, 1);
-    if (e == cudaSuccess && !S->d_rows) e = dalloc(&S->d_rows, (size_t)S->cap * k);
-    if (e == cudaSuccess && !S->d_wave) e = dalloc(&S->d_wave, (size_t)S->cap);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_work, 0, 16, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_count, 0, 8, st);
-    if (e != cudaSuccess) {
-      release();
-      return set_error(e == cudaErrorMemoryAllocation ? KCLPP_ERR_NOMEM : KCLPP_ERR_CUDA, "sampling: %s",
-                       cudaGetErrorString(e));
-    }
+  // One run of the kernels into S's buffers; *got receives the rows counted.
+  auto draw = [&](unsigned long long *wave_at, unsigned long long *got) -> kclpp_status {
+    SCUDA(cudaMemsetAsync(d_work, 0, 16, st));
+    SCUDA(cudaMemsetAsync(d_count, 0, 8, st));
     SampleArgs a{};
     a.off = graph_dev_offsets(S->g);
     a.cols = graph_dev_cols(S->g);
@@ -613,17 +620,29 @@ kclpp_status sample(kclpp_ctx *c, kclpp_sampling *S) {
     a.wave = S->d_wave;
     a.cap = S->cap;
     a.count = d_count;
+    a.wave_at = wave_at;
     a.bit_rows = graph_dev_bit_rows(S->g);
     a.bits = graph_dev_bits(S->g);
-    status = launch_k(k, c, S, a, graph_dev_count_roots(S->g), bounds, dmax, d_work);
-    if (status != KCLPP_OK) break;
-    unsigned long long got = 0;
-    e = cudaMemcpyAsync(&got, d_count, 8, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    STRY(launch_k(k, c, S, a, graph_dev_count_roots(S->g), bounds, dmax, d_work));
+    SCUDA(cudaMemcpyAsync(got, d_count, 8, cudaMemcpyDeviceToHost, st));
+    SCUDA(cudaStreamSynchronize(st));
+    return KCLPP_OK;
+  };
+  kclpp_status status = KCLPP_OK;
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    cudaError_t e = cudaSuccess;
+    if (e == cudaSuccess && !d_work) e = dalloc(&d_work, 4);
+    if (e == cudaSuccess && !d_count) e = dalloc(&d_count, 1);
+    if (e == cudaSuccess && !S->d_rows) e = dalloc(&S->d_rows, (size_t)S->cap * k);
+    if (e == cudaSuccess && !S->d_wave) e = dalloc(&S->d_wave, (size_t)S->cap);
     if (e != cudaSuccess) {
-      status = set_error(KCLPP_ERR_CUDA, "sampling: %s", cudaGetErrorString(e));
-      break;
+      release();
+      return set_error(e == cudaErrorMemoryAllocation ? KCLPP_ERR_NOMEM : KCLPP_ERR_CUDA, "sampling: %s",
+                       cudaGetErrorString(e));
     }
+    unsigned long long got = 0;
+    status = draw(nullptr, &got);
+    if (status != KCLPP_OK) break;
     S->sampled = got;
     if (got <= S->cap) break;
     if (attempt == 1) {
@@ -636,8 +655,13 @@ kclpp_status sample(kclpp_ctx *c, kclpp_sampling *S) {
     S->d_wave = nullptr;
     S->cap = got;
   }
+  if (status == KCLPP_OK)
+    status = group_by_wave(c, S, [&](unsigned long long *wave_at) {
+      unsigned long long none = 0;
+      return draw(wave_at, &none);
+    });
   release();
-  return status == KCLPP_OK ? group_by_wave(c, S) : status;
+  return status;
 }
 
 kclpp_status check_ctx(kclpp_ctx *c, const kclpp_sampling *S) {
