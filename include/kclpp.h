@@ -337,6 +337,9 @@ kclpp_status kclpp_densest_exact(const kclpp_edge_list *el, int k, kclpp_exact_i
  * Where the loads do not settle "inside" within max_passes and G[S] has at
  * most 2e7 k-cliques, the host max-flow (kclpp_densest_exact) on G[S] decides
  * it, as the reference falls back to its max-flow (kCDensestMem.c:434-467).
+ * When that max-flow finds a denser subset of S, max_passes more shared-load
+ * passes from r give a second candidate, which takes S's place if it is
+ * certified (:478-530 go on with their passes); otherwise info describes S.
  * members (n entries, or NULL) gets S's vertices. */
 typedef struct {
   uint32_t n;              /* vertices of the candidate S                      */

@@ -2337,10 +2337,13 @@ cudaError_t launch_tier(const TierLaunch &t, dev::PassArgs a, cudaStream_t st) {
     e = prepare(fn, lc, nw * 32, sm, &per_sm);
     if (e != cudaSuccess) return e;
     // Shared loads: every stream in flight is blind to the others, so more of
-    // them at once cost passes.  24 warps an SM instead of what fits: a planted
-    // RMAT-13 at k = 5 takes 81 to 83 passes to a certified gap (92 to 101), a
-    // planted RMAT-12 at k = 3 is certified from 64 passes in 60 of 60 runs (58),
-    // and its pass takes 96 us (129).
+    // them at once cost passes.  A launch takes at most 24 warps an SM (20 of
+    // width 20, 16 of width 16) instead of what fits; the groups of a pass may
+    // run side by side, so the pass as a whole can hold more.  A planted RMAT-13
+    // at k = 5 takes 81 to 83 passes to a certified gap (92 to 101); a planted
+    // RMAT-12 at k = 3 has its densest set first after 64 passes in 336 of 360
+    // runs (308) of passes alone, in 208 of 300 when each run is certified, and
+    // its pass takes 96 us (129).
     if (MODE == MODE_SEQ && a.shared_loads) per_sm = std::min(per_sm, std::max(1, 24 / nw));
     fn<<<persistent_grid(per_sm, t, 1, t.active != nullptr), nw * 32, sm, st>>>(a);
     return cudaGetLastError();
