@@ -431,7 +431,8 @@ static kclpp_status build_schedule(kclpp_ctx *c, kclpp_graph *g) {
 // id range it spans (two words per edge): inducing a root's rows asks such a
 // vertex about 32 members at a time, where walking its list costs a look-up per
 // edge and mostly misses.  At most 8 bytes per edge; sparser lists stay short
-// for the ids they span and are walked.  Needs d_off and d_cols.
+// for the ids they span and are walked, and so is every list where the device
+// has no room for the rows: they come after all that a graph cannot do without.
 static kclpp_status upload_bit_rows(kclpp_ctx *c, kclpp_graph *g) {
   const HostDag &D = g->dag;
   std::vector<uint4> rows(D.n);
@@ -447,8 +448,16 @@ static kclpp_status upload_bit_rows(kclpp_ctx *c, kclpp_graph *g) {
     words += w;
   }
   if (!words) return KCLPP_OK;
-  KCL_TRY(dalloc(&g->d_bit_rows, D.n));
-  KCL_TRY(dalloc(&g->d_bits, words));
+  cudaError_t room = cudaMalloc((void **)&g->d_bit_rows, (size_t)D.n * sizeof(uint4));
+  if (room == cudaSuccess) room = cudaMalloc((void **)&g->d_bits, words * 4);
+  if (room == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    cudaFree(g->d_bit_rows);
+    g->d_bit_rows = nullptr;
+    g->d_bits = nullptr;
+    return KCLPP_OK;
+  }
+  KCL_CUDA(room);
   KCL_CUDA(cudaMemcpyAsync(g->d_bit_rows, rows.data(), (size_t)D.n * sizeof(uint4), cudaMemcpyHostToDevice, c->stream));
   KCL_CUDA(cudaMemsetAsync(g->d_bits, 0, words * 4, c->stream));
   k_bit_rows<<<std::min(blocks_for(D.n, 8), c->num_sms * 8), 256, 0, c->stream>>>(g->d_off, g->d_cols, g->d_bit_rows,
@@ -474,7 +483,6 @@ static kclpp_status upload_graph(kclpp_ctx *c, kclpp_graph *g) {
       for (uint64_t e = D.off[s]; e < D.off[s + 1]; ++e) src[e] = s;
     KCL_CUDA(cudaMemcpyAsync(g->d_src, src.data(), D.m() * 4, cudaMemcpyHostToDevice, c->stream));
     KCL_CUDA(cudaStreamSynchronize(c->stream));
-    KCL_TRY(upload_bit_rows(c, g));
   }
   KCL_TRY(build_schedule(c, g));
   const size_t n1 = (size_t)D.n + 1;
@@ -483,6 +491,7 @@ static kclpp_status upload_graph(kclpp_ctx *c, kclpp_graph *g) {
   KCL_TRY(dalloc(&g->d_rho, n1));
   KCL_TRY(dalloc(&g->d_level, n1));
   KCL_TRY(dalloc(&g->d_scalar, 4));
+  if (D.m()) KCL_TRY(upload_bit_rows(c, g));
   KCL_CUDA(cudaStreamSynchronize(c->stream));
   return KCLPP_OK;
 }
