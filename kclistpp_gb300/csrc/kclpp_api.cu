@@ -554,10 +554,15 @@ static std::vector<TierInfo> launch_plan(const std::vector<TierInfo> &tiers, con
 }
 
 // Smallest root that idle CTAs join.  Joining means building the root's rows
-// again, which pays where its streams cost more: never at k = 3 (RMAT-17: 680
-// us a pass without, 912 with), from 128 members at k = 4 (a core of out-degree
-// 371: 660 us without, 482 with; 60,000 vertices, out-degree <= 128: 240 and
-// 290), from 32 beyond (a core of out-degree 120 at k = 5: 1656 and 779).
+// again, which pays where its streams cost more.  Never at k = 3, however dense
+// (us a pass without and with, from 33 members): a G(n, p) of 600 vertices at
+// 0.9, out-degree <= 518, 141 and 388; of 1000 at 0.9, <= 868, 527 and 686; the
+// same in a sparse graph of 60,000, 583 and 738; an RMAT-18 core, <= 372, 169
+// and 333; RMAT-17, 713 and 854; thresholds of 257 to 513 lie between.  From 129
+// members at k = 4 (from 129, from 33, never): G(300, 0.9) 672, 684, 1692;
+// G(600, 0.9) 2800, 2802, 4189; the RMAT-18 core 638, 599, 712; 60,000 vertices
+// with communities, <= 124, 254, 305, 254; RMAT-17 1296, 1298, 1215.  From 33
+// beyond (a core of out-degree 120 at k = 5: 779, never 1656).
 static uint32_t steal_from(int mode, int k) {
   return mode != dev::MODE_SEQ ? 0u : k == 3 ? UINT32_MAX : k == 4 ? 129u : 33u;
 }

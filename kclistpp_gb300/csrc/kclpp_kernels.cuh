@@ -28,7 +28,11 @@
 //              (credits g) iff cur[v] >= c0 + (failures before it); the failure
 //              mask is the unique fixed point of that rule and is found by
 //              iterating ballots (lane i is final after i+1 rounds, so the loop
-//              is bounded by 33 rounds).
+//              is bounded by 33 rounds).  With rows in shared memory the last
+//              two levels are first settled 32 vertices at a time by counting
+//              (TinyStream: at most 64 candidates, in registers; PairLevel:
+//              the others), and only a group whose comparisons can still
+//              change runs its chains one after another.
 //
 // Set iteration always walks a copy of the set (`it`) and intersects with the
 // unmodified set, because the child set of u is P ∩ N+(u) over all of P.
@@ -833,32 +837,6 @@ __device__ __forceinline__ typename VA::T value_of(int x, const VA &va, int lane
   return __shfl_sync(KCL_FULL, v, x & 31);
 }
 
-// The last two levels of a stream, at once: for u in P ascending, the chain
-// over V = P ∩ row(u) (kCDensestNoAtom.c:173-188), values in 32 bits.
-//
-// What bounds these levels is instruction issue, and a walk over the words of
-// every V spends it on lanes without a candidate and on candidates whose fate
-// is known.  A member whose value is at or above c + |P| (|P| - 1) / 2 -- c
-// plus every clique of the call -- can never be below a prefix value: it falls
-// every time and never changes.  Only the others, I, are followed, compacted
-// 32 to a slot.  The members u are taken 32 at a time (lane g: u_g, with
-// tot_g = |V|).
-//
-// A group whose comparisons cannot change their outcome while it runs is
-// settled by counting.  Inside the group i's value stays in [v_i, v_i + S_i],
-// S_i = 32 + (i in the group: tot_i), and the prefix value in [c, c + sum
-// tot].  If every i lies wholly below c (class L) or at or above c + sum tot,
-// every chain of a u outside L gives its unit to exactly the members of V in
-// L, the rest falls to the prefix; a u in L is its own prefix (value v_u, up
-// to v_u + S_u) and is compared the same way with its V.  T_i, in i's lane,
-// has bit g set iff i is in u_g's V, so these are popcounts.  When any two of
-// the compared ranges overlap, the group's chains run one after another.
-//
-// Measured on a trimmed RMAT-18 core (233 K edges, k = 4, loads of 4 passes):
-// 94 % of the groups settle; a pass 3.87 -> 1.47 ms against the word-at-a-time
-// chain alone.  From zero, where nothing settles (k = 5, RMAT-15 with planted
-// communities), 15.0 -> 11.9 ms.  At most 40 registers at k = 4 (48 warps per
-// SM): at 80 (24 warps) the same pass took 2.16 ms.
 // Values of a root as 32-bit offsets from its smallest, capped here (the Seq
 // kernel with rows in shared memory).
 constexpr uint32_t kRelCap = 0x7ffffff0u;
@@ -1094,6 +1072,33 @@ __device__ __forceinline__ int list_members(uint32_t P, uint16_t *list, int lane
   return np;
 }
 
+// The last two levels of a stream, at once: for u in P ascending, the chain
+// over V = P ∩ row(u) (kCDensestNoAtom.c:173-188), values in 32 bits.
+//
+// What bounds these levels is instruction issue, and a walk over the words of
+// every V spends it on lanes without a candidate and on candidates whose fate
+// is known.  A member whose value is at or above c + |P| (|P| - 1) / 2 -- c
+// plus every clique of the call -- can never be below a prefix value: it falls
+// every time and never changes.  Only the others, I, are followed, compacted
+// 32 to a slot.  The members u are taken 32 at a time (lane g: u_g, with
+// tot_g = |V|).
+//
+// A group whose comparisons cannot change their outcome while it runs is
+// settled by counting.  Inside the group i's value stays in [v_i, v_i + S_i],
+// S_i = 32 + (i in the group: tot_i), and the prefix value in [c, c + sum
+// tot].  If every i lies wholly below c (class L) or at or above c + sum tot,
+// every chain of a u outside L gives its unit to exactly the members of V in
+// L, the rest falls to the prefix; a u in L is its own prefix (value v_u, up
+// to v_u + S_u) and is compared the same way with its V.  T_i, in i's lane,
+// has bit g set iff i is in u_g's V, so these are popcounts.  When any two of
+// the compared ranges overlap, the group's chains run one after another.
+//
+// Measured on a trimmed RMAT-18 core (233 K edges, k = 4, loads of 4 passes):
+// 94 % of the groups settle; a pass 3.87 -> 1.47 ms against the word-at-a-time
+// chain alone.  From zero, where nothing settles (k = 5, RMAT-15 with planted
+// communities), 15.0 -> 11.9 ms.  At most 40 registers at k = 4 (48 warps per
+// SM): at 80 (24 warps) the same pass took 2.16 ms.
+//
 // ACC: the values are the root's own (shared by its streams, read only) and
 // increments go to acc; else the values are the stream's and are updated.
 template <bool ACC>
@@ -1921,10 +1926,11 @@ __device__ __forceinline__ uint32_t find_victim(const PassArgs &a, int need, uin
   return s_who[__ffs(__ballot_sync(KCL_FULL, mine == all)) - 1];
 }
 
-// Register budget of a tier M / L kernel, as CTAs of the widest launch that
-// must fit one SM: two for the shallow recursions (the Seq kernel then keeps
-// <= 42 registers a thread at k = 3, 4; the counting kernels <= 32 at k <= 4
-// and <= 42 at k = 5 with 24-warp CTAs), one for the deeper ones, which would
+// Register budget of a tier M / L kernel, as CTAs of the widest launch
+// (warps_m) that must fit one SM: two for the Seq kernels, whose widest launch
+// narrows as k grows (40 registers a thread at k <= 4, 64 at k = 5, 6, 80
+// beyond), and for the shallow counting kernels (<= 32 at k <= 4, <= 42 at
+// k = 5 with 24-warp CTAs); one for the deeper counting kernels, which would
 // otherwise spill.
 template <int MODE, int K>
 constexpr int min_ctas_m() { return MODE == MODE_SEQ || K <= 5 ? 2 : 1; }
