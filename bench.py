@@ -19,9 +19,9 @@ root edges of the same workload.
 The graph preparation (generation, trim, DAG) is not timed; the trim counts
 cliques on the GPU in both arms.
 
-The JSON line also carries: the pass-level roofline (the reference's
-per-root-edge gather bytes over the Seq pass time, against the measured HBM
-copy bandwidth), the host-buffer run through the C ABI (`e2e`, the same
+The JSON line also carries: the pass-level roofline (warp instructions of the
+Seq pass over its time, against the issue peak; beside it the reference's
+per-root-edge gather bytes over the same time), the host-buffer run through the C ABI (`e2e`, the same
 passes from the same state), the CPU port's rate (`cpu_baseline`), clocks
 sampled during the timed region, and `convergence`: wall time to a certified
 1 % density gap on a held-out RMAT-16 graph with planted communities (k = 5)
@@ -899,46 +899,40 @@ def main() -> None:
 
     # Roofline of the dominant kernel: one pass of the mode that takes the most
     # time (its root groups run as concurrent launches of one kernel, so the
-    # pass, timed on the launching stream, is the unit).  Bytes: the per-root-
-    # edge gathers of the reference's MakeSubgraph over every root edge.
+    # pass, timed on the launching stream, is the unit).  The dense core is L2-
+    # resident and every scheduler issues most cycles, so the roof is instruction
+    # issue: SMs x 4 schedulers x one warp instruction per cycle at the sampled
+    # SM clock; the instructions are the committed counters of this workload
+    # (without them there is no fraction).  Beside it, as a measure of work and
+    # not of traffic, the reference's per-root-edge gathers of MakeSubgraph.
     peak, peak_kind = measured_peaks()
     roofline = None
     if pass_ms and stats["ref_equiv_bytes_per_pass"]:
         md = max(pass_ms, key=pass_ms.get)
+        st = stats_seq if md == "seq" else stats
+        mhz = (clk or {}).get("sm_mhz") or 2070.0
+        sms = torch.cuda.get_device_properties(local).multi_processor_count
+        ipeak = sms * 4 * mhz * 1e6
+        wi = profiled("warp_inst_per_pass", md, a)
+        iach = wi / (pass_ms[md] / 1000.0) if wi else None
         bpp = stats["ref_equiv_bytes_per_pass"]
         achieved = bpp / (pass_ms[md] / 1000.0) / 1e9
-        st = stats_seq if md == "seq" else stats
-        roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                    "traffic": profiled("dram_bytes_per_pass", md, a), "kernel": f"{'seq' if md == 'seq' else 'order'} pass "
+        roofline = {"bound": "issue", "achieved": iach, "peak": ipeak, "unit": "warp inst/s",
+                    "frac": iach / ipeak if wi else None, "warp_inst_per_pass": wi, "sm_mhz": mhz, "sms": sms,
+                    "kernel": f"{'seq' if md == 'seq' else 'order'} pass "
                     f"(tier_m_kernel/tier_s_kernel, {len(st['tiers'])} concurrent root groups)",
-                    "bytes_per_launch": bpp,
-                    "impl_bytes_per_launch": sum(v["impl_bytes"] for v in st["tiers"].values()),
-                    "avg_launch_ms": pass_ms[md], "peak_source": f"{peak_kind} hbm_gbs",
-                    "pass_ms": pass_ms,
-                    "note": "bytes = reference-equivalent bytes: the reference's per-root-edge gathers "
-                            "(MakeSubgraph, kCDensestNoAtom.c:86-113) over every root edge of the pass; this "
-                            "implementation reads impl_bytes of them (one induction per root vertex) and the DAG "
-                            "stays in L2, so DRAM traffic (from the committed ncu summary) is far below and frac "
-                            "can exceed 1: it rates the work those bytes stand for, not traffic; the pass is bound "
-                            "by instruction issue (see issue)",
-                    "step_achieved": bpp * len(modes) / (ms / 1000.0) / 1e9}
-        roofline["step_frac"] = roofline["step_achieved"] / peak
-        # What actually bounds the pass: the dense core is L2-resident and the
-        # kernel issues instructions on every scheduler most cycles, so the
-        # instruction-issue roof (152 SMs x 4 schedulers x one warp instruction
-        # per cycle at the sampled SM clock) is the one to read the pass
-        # against; the bytes above are the reference-equivalent work figure.
-        wi = profiled("warp_inst_per_pass", md, a)
-        if wi:
-            mhz = (clk or {}).get("sm_mhz") or 2070.0
-            sms = torch.cuda.get_device_properties(local).multi_processor_count
-            ipeak = sms * 4 * mhz * 1e6
-            iach = wi / (pass_ms[md] / 1000.0)
-            roofline["issue"] = {"bound": "issue", "achieved": iach, "peak": ipeak, "unit": "warp inst/s",
-                                 "frac": iach / ipeak, "warp_inst_per_pass": wi, "sm_mhz": mhz, "sms": sms,
-                                 "l2_bytes_per_pass": profiled("l2_bytes_per_pass", md, a),
-                                 "dram_bytes_per_pass": profiled("dram_bytes_per_pass", md, a),
-                                 "source": os.path.relpath(PASS_COUNTERS, ROOT)}
+                    "avg_launch_ms": pass_ms[md], "pass_ms": pass_ms,
+                    "l2_bytes_per_pass": profiled("l2_bytes_per_pass", md, a),
+                    "traffic": profiled("dram_bytes_per_pass", md, a),
+                    "source": os.path.relpath(PASS_COUNTERS, ROOT) if wi else None,
+                    "reference_bytes": {
+                        "bytes_per_pass": bpp, "rate": achieved, "step_rate": bpp * len(modes) / (ms / 1000.0) / 1e9,
+                        "unit": "GB/s", "hbm_gbs": peak, "hbm_source": f"{peak_kind} hbm_gbs",
+                        "impl_bytes_per_pass": sum(v["impl_bytes"] for v in st["tiers"].values()),
+                        "note": "the reference's per-root-edge gathers (MakeSubgraph, kCDensestNoAtom.c:86-113) "
+                                "over every root edge, by the pass time: the rate of the work those bytes stand "
+                                "for, above the HBM rate because they are not moved (one induction per root "
+                                "vertex, the DAG in L2)"}}
     kernels = [{**p, "avg_ms": p["ms"] / max(1, p["launches"])} for p in prof]
 
     # ---- end to end through the C ABI with host buffers -------------------------------
