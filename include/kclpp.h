@@ -159,7 +159,8 @@ kclpp_status kclpp_count_edges(kclpp_ctx *ctx, const kclpp_graph *g, uint32_t nu
  * CTAs are working on.  Defaults: tier_s_max 64, tier_s_max_seq 16, splits
  * 256 / 512, Seq stealing on (for roots worth it at the pass's k), counting stealing off, 4 waves, widths 0 (auto),
  * concurrent groups on.  At its default, a tier S bound follows k: the counting
- * kernels at k >= 5 give roots of 33..64 a CTA, and the Seq kernel at k <= 4
+ * kernels give roots of 33..64 a CTA (Sim and PAVA at k >= 5, k-clique degrees at
+ * k = 5 and, with counting stealing on, beyond), and the Seq kernel at k <= 4
  * (but for KCLPP_SEQ_SHARED) gives a warp to a group whose roots have at most
  * 32.  Any other bound is kept at every k. */
 typedef struct {

@@ -519,14 +519,19 @@ struct Exec {
 //    for the root edges): 20,000 vertices of out-degree <= 29 at k = 4, 149 us
 //    a pass apart, 89 together; 10,000 with 632 such roots 53 and 46.  From
 //    k = 5 on a lane's stream is long, and the CTA stays the better one.
-//  * Counting, k >= 5: warp-per-root roots above 32 members, whose rows a lane
-//    counts alone, go to a CTA: a core of out-degree 120 at k = 5, 424 us a Sim
-//    pass with the warp, 228 with the CTA; at k = 4 there is no difference.
+//  * Sim and the prefix counts at k >= 5, clique degrees at k = 5: warp-per-root
+//    roots above 32 members, whose rows a lane counts alone, go to a CTA: a core
+//    of out-degree 120 at k = 5, 424 us a Sim pass with the warp, 228 with the
+//    CTA; at k = 4 there is no difference.  Clique degrees beyond k = 5, whose
+//    CTA walks symmetric rows a word per lane, only where other CTAs may join:
+//    20,000 vertices of out-degree <= 46 at k = 7 take 8.4 ms with the warp and
+//    18.8 with the CTA, a G(60, 0.9) 15.2 and 31.4 (10.5 with stealing).
 // Both are what a tier S bound left at its default means; a program that sets
 // another bound has exactly that one, at every k.
 static std::vector<TierInfo> launch_plan(const std::vector<TierInfo> &tiers, const kclpp_schedule &sp, int mode,
                                          int k) {
   if (mode == dev::MODE_SEQ ? sp.tier_s_max_seq != kTierSMaxSeq : sp.tier_s_max != kTierSMax) return tiers;
+  const bool cta32 = mode == dev::MODE_ORDER ? k >= 5 : mode == dev::MODE_COUNT && (sp.steal_count ? k >= 5 : k == 5);
   std::vector<TierInfo> plan;
   for (TierInfo t : tiers) {
     const TierInfo *prev = plan.empty() ? nullptr : &plan.back();
@@ -537,7 +542,7 @@ static std::vector<TierInfo> launch_plan(const std::vector<TierInfo> &tiers, con
                prev->offset + prev->count == t.offset) {
       plan.back().count += t.count;
       continue;
-    } else if (mode != dev::MODE_SEQ && k >= 5 && t.tier == 0 && t.over32) {
+    } else if (cta32 && t.tier == 0 && t.over32) {
       TierInfo hi = t;
       hi.tier = 1;
       hi.bucket = 0;

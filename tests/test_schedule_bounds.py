@@ -20,8 +20,12 @@ def _clique(n):
 def test_kernels_launched(tmp_path):
     fake_cuda.run(tmp_path, """
         from tests.test_schedule_bounds import _clique
-        def route(n, k, seq, smax):
+        def route(n, k, seq, smax, steal=0):
             g = K.build_graph(ctx, K.EdgeList.from_pairs(_clique(n)))
+            if steal:
+                sp = K.get_schedule(g)
+                sp.steal_count = 1
+                K.set_schedule(g, sp)
             if smax is not None:
                 sp = K.get_schedule(g)
                 if seq: sp.tier_s_max_seq = smax
@@ -37,7 +41,8 @@ def test_kernels_launched(tmp_path):
             for smax, want in ((1, [1, 1]), (8, [1, 1]), (15, [1, 1]), (17, [1, 1]), (29, [1, 0]), (64, [1, 0])):
                 assert route(30, k, True, smax) == want, (k, smax)
             # out-degrees 1..59
-            assert route(60, k, False, None) == ([1, 0] if k <= 4 else [1, 1]), k
+            assert route(60, k, False, None) == ([1, 1] if k == 5 else [1, 0]), k
+            assert route(60, k, False, None, steal=1) == ([1, 0] if k <= 4 else [1, 1]), k
             for smax, want in ((1, [1, 1]), (32, [1, 1]), (58, [1, 1]), (59, [1, 0]), (63, [1, 0])):
                 assert route(60, k, False, smax) == want, (k, smax)
         """)
