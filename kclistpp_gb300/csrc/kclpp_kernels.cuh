@@ -53,6 +53,7 @@ namespace dev {
 // Tier S: one warp per root, d <= 64, 64-bit rows, one lane per row / edge.
 constexpr int kSMaxD = 64;
 constexpr int kSDl = kSMaxD + 1;  // per-lane delta stride
+constexpr int kSFew = 32;         // most members of a root whose rows are built in registers
 
 // A root's members by id: an open-addressing table of 2^bits slots, at most a
 // quarter full up to 512 members and half full beyond.  An id's home is the
@@ -255,7 +256,59 @@ __global__ void __launch_bounds__(kWarpsS * 32) tier_s_kernel(PassArgs a) {
     }
     for (int i = lane; i < kSMaxD; i += 32) sm.rows[i] = 0;
     __syncwarp();
-    if (K >= 3) {
+    if (K >= 3 && d <= kSFew) {
+      // Rows as below, of at most a word: row `lane` in a register.  A member
+      // with a bitmap row is asked about the ones before it; another's out-list
+      // is merged with the members, four neighbours at a time.  Instruction
+      // issue over many small roots bounds this, and the table, its look-ups and
+      // a step per member without a row cost more than these roots hold: 400,000
+      // vertices of out-degree <= 37, a k = 3 Sim pass 427 us with the table, 322
+      // so; an RMAT-18 graph, whose hubs the bitmap rows answer for, 1059 and 963
+      // (merging every list: 1407).
+      const uint32_t y = lane < d ? sm.list[lane] : 0u;
+      const bool row_of = lane > 0 && lane < d;
+      const uint4 b = row_of ? bit_row(a, y) : make_uint4(0, 0, 0, 0);
+      const uint64_t e0 = row_of ? a.off[y] : 0ull, xe = row_of ? a.off[y + 1] : 0ull;
+      uint32_t row = 0;
+      for (uint32_t has = __ballot_sync(KCL_FULL, row_of && b.x != kNoBitRow); has; has &= has - 1) {
+        const int i = __ffs((int)has) - 1;
+        const uint32_t bo = __shfl_sync(KCL_FULL, b.x, i), bf = __shfl_sync(KCL_FULL, b.y, i);
+        const uint32_t bs = __shfl_sync(KCL_FULL, b.z, i);
+        const uint32_t m = __ballot_sync(KCL_FULL, lane < i && bit_at(a, bo, bf, bs, y));
+        if (lane == i) row = m;
+      }
+      if (row_of && b.x == kNoBitRow) {
+        int j = 0;
+        uint32_t at = sm.list[0];
+        for (uint64_t e = e0; e < xe && j < lane; e += 4) {
+          uint32_t z[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) z[q] = e + q < xe ? a.cols[e + q] : 0xffffffffu;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            while (j < lane && at < z[q]) at = sm.list[++j];
+            if (j < lane && at == z[q]) row |= 1u << j;
+          }
+        }
+      }
+      if constexpr (MODE == MODE_SEQ) {
+        if (lane < d) sm.rows[lane] = row;
+      } else {
+        uint32_t full = row;  // symmetric: the column off the others' rows
+        for (int g = 1; g < d; ++g) {
+          const uint32_t m = __shfl_sync(KCL_FULL, row, g);
+          if (lane < g && ((m >> lane) & 1u)) full |= 1u << g;
+        }
+        if constexpr (MODE == MODE_ORDER) {  // by key rank, upward
+          uint32_t up = 0;
+          for (uint32_t it = __shfl_sync(KCL_FULL, full, lane < d ? sm.inv[lane] : 0); it; it &= it - 1)
+            up |= 1u << sm.rank[__ffs((int)it) - 1];
+          full = lane < d ? up & ~((2u << lane) - 1u) : 0u;
+        }
+        if (lane < d) sm.rows[lane] = full;
+      }
+      __syncwarp();
+    } else if (K >= 3) {
       // Row i: out-neighbours of list[i] inside N+(s) (MakeSubgraph's induced
       // adjacency, :104-113).  A member with a bitmap row is asked about every
       // member before it at once, a lane each; the others' out-lists are
