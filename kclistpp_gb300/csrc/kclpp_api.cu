@@ -61,7 +61,8 @@ struct kclpp_ctx {
   unsigned char *pin = nullptr;  // pinned staging of host-vector calls (Staged)
   size_t pin_used = 0;
 };
-constexpr size_t kPinBytes = 1 << 20;
+constexpr size_t kPinBytes = 1 << 19;
+constexpr size_t kStageMax = 192 << 10;  // longest vector that goes through it (Staged)
 
 static cudaEvent_t take_event(kclpp_ctx *c) {
   if (!c->event_pool.empty()) {
@@ -206,9 +207,12 @@ static kclpp_status check_err(kclpp_ctx *c) {
 }
 
 // Copies of a call that takes and returns host vectors, through the context's
-// pinned megabyte where they fit: a copy to or from pageable memory waits in the
-// driver, two or three times a call (the triangle counts of 10,000 vertices: 59
-// us with direct copies, 54 staged).  Larger vectors are copied directly.
+// pinned memory where they are short: a copy to or from pageable memory waits in
+// the driver, two or three times a call (the triangle counts of 10,000 vertices:
+// 50 us with direct copies, 44 staged).  Vectors beyond kStageMax are copied
+// directly: staging adds a pass over them that the driver's own copy overlaps
+// (the Sim counts of 127,000 vertices, 1 MB each way: 191 us with one of the two
+// staged, 161 direct; of 30,000, 240 KB: 81 either way).
 // finish() ends the call: it reads the status word, waits, and hands the results
 // over, so that a call that fails leaves the caller's vectors as they were.
 class Staged {
@@ -259,7 +263,7 @@ class Staged {
   };
   unsigned char *room(size_t bytes) {
     const size_t at = (c_->pin_used + 15) & ~(size_t)15;
-    if (!c_->pin || at + bytes > kPinBytes - 16) return nullptr;
+    if (!c_->pin || bytes > kStageMax || at + bytes > kPinBytes - 16) return nullptr;
     c_->pin_used = at + bytes;
     return c_->pin + at;
   }

@@ -1,7 +1,6 @@
 """A call whose device status word reports an error leaves the caller's host
-vectors as they were, at sizes that the pinned staging holds (up to 131070
-entries, 65535 for a vector both read and written) and beyond.  On the host, with
-a status word that the test sets (tests/fake_cudart.c)."""
+vectors as they were, at sizes that go through the pinned staging (up to 24576
+entries) and beyond.  On the host, with a status word that the test sets (tests/fake_cudart.c)."""
 from tests import fake_cuda
 
 
@@ -10,7 +9,7 @@ def test_vectors_stay_as_they_were(tmp_path):
         L, u64 = K._lib, C.POINTER(C.c_uint64)
         def u(a): return a.ctypes.data_as(u64)
         def d(a): return a.ctypes.data_as(C.POINTER(C.c_double))
-        for n in (10, 65000, 100000, 131070, 131071, 200000):
+        for n in (10, 24575, 24576, 24577, 65000, 100000, 131070, 131071, 200000):
             off = np.concatenate([[0], np.arange(n)]).astype(np.uint64)    # a path
             g = K.graph_from_csr(ctx, off, np.arange(n - 1).astype(np.uint32))
             assert g.n == n
