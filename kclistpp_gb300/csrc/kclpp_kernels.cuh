@@ -1712,6 +1712,27 @@ __device__ __forceinline__ bool stream_on_rel(const Bits<1> &C, uint32_t nc, int
 constexpr int kTaskBits = 20;  // 2048 sub-tasks and one overshoot per warp of 2048 CTAs
 constexpr uint32_t kTaskMask = (1u << kTaskBits) - 1u;
 
+// A stream on 64-bit values at k >= 6 (its values differ by 2^31 or more).  A
+// function of its own, so that its recursion does not share its registers with
+// what the other streams keep: loads spread over 2^40, us a pass inlined and so,
+// planted RMAT-12 at k = 6 2906 and 2482, Chung-Lu 3,000 at k = 8 4441 and 3295;
+// no difference for loads within 2^31.
+template <int K>
+__device__ __noinline__ void stream_wide(uint32_t word, int g0, const uint32_t *rows, const unsigned long long *base,
+                                         uint32_t *cur, unsigned long long *acc, int lane, uint32_t *err) {
+  Bits<1> C;
+  C.w[0] = word;
+  for_members<1>(C, lane, [&](int i) { cur[i] = 0; });
+  const Vals64<true> va{base, cur};
+  const unsigned long long c0 = base[g0];
+  const unsigned long long c1 = seq_rec<K - 2, 1, Vals64<true>, false>(C, c0, rows, va, 0u, lane, err);
+  for_members<1>(C, lane, [&](int i) {
+    const uint32_t delta = cur[i];
+    if (delta) shared_add(&acc[i], delta);
+  });
+  if (lane == 0 && c1 != c0) shared_add(&acc[g0], c1 - c0);
+}
+
 // Every root-edge stream of the current root, the warp taking streams from
 // the root's shared counter (largest candidate sets first); increments go to
 // the CTA's acc[] (kCDensestNoAtom.c:270-295 per root edge).
@@ -1747,6 +1768,10 @@ __device__ __forceinline__ void seq_streams(uint32_t *next, int d, const uint32_
       const uint32_t nc = __reduce_add_sync(KCL_FULL, (uint32_t)__popc(C.w[0]));
       if (nc < (uint32_t)(K - 2)) continue;
       if (stream_on_rel<K>(C, nc, g0, rows, rel, cur, acc, pair, lane, err)) continue;
+      if constexpr (K >= 6) {
+        stream_wide<K>(C.w[0], g0, rows, base, cur, acc, lane, err);
+        continue;
+      }
     }
     bool r32 = false;
     unsigned long long off = 0, cap = 0;
