@@ -642,6 +642,7 @@ static kclpp_status run_tiers(kclpp_ctx *c, kclpp_graph *g, int mode, int k, dev
     tl.task_next = task + (t.offset - base);
     tl.active = steal && t.tier > 0 && t.dmax >= steal_min ? registry + i * kActiveSlots : nullptr;
     tl.num_sms = c->num_sms;
+    tl.streams = g->dag.m();
     tl.max_grid = t.tier == 2 ? g->slab_ctas : 0;
     tl.warps = t.bucket < 0 ? 0 : (int)(mode == dev::MODE_SEQ ? g->sp.seq_warps[t.bucket] : g->sp.count_warps[t.bucket]);
     cudaError_t e = cudaSuccess;

@@ -133,6 +133,7 @@ struct TierLaunch {
   int num_sms;
   int max_grid;      // upper bound on CTAs (tier L: CTAs the row slab holds)
   int warps;         // tiers M / L: warps per CTA (0 = the most resident warps)
+  uint64_t streams;  // root edges of the pass (shared loads)
 };
 cudaError_t launch_count(int k, const TierLaunch &t, dev::PassArgs a, cudaStream_t st);
 cudaError_t launch_order(int k, const TierLaunch &t, dev::PassArgs a, cudaStream_t st);

@@ -2420,15 +2420,20 @@ cudaError_t launch_tier(const TierLaunch &t, dev::PassArgs a, cudaStream_t st) {
     const size_t sm = layout_m(MODE, K, t.dmax, nw, true).total;
     e = prepare(fn, lc, nw * 32, sm, &per_sm);
     if (e != cudaSuccess) return e;
-    // Shared loads: every stream in flight is blind to the others, so more of
-    // them at once cost passes.  A launch takes at most 24 warps an SM (20 of
-    // width 20, 16 of width 16) instead of what fits; the groups of a pass may
-    // run side by side, so the pass as a whole can hold more.  A planted RMAT-13
-    // at k = 5 takes 81 to 83 passes to a certified gap (92 to 101); a planted
-    // RMAT-12 at k = 3 has its densest set first after 64 passes in 336 of 360
-    // runs (308) of passes alone, in 208 of 300 when each run is certified, and
-    // its pass takes 96 us (129).
-    if (MODE == MODE_SEQ && a.shared_loads) per_sm = std::min(per_sm, std::max(1, 24 / nw));
+    // Shared loads: every stream in flight is blind to the others, so that too
+    // large a share of a pass at once costs passes.  A launch takes at most a
+    // 32nd of the root edges, but 24 warps an SM at least (20 of width 20, 16 of
+    // width 16); the groups of a pass may run side by side, so the pass as a
+    // whole can hold more.  Passes to a certified 1 % gap (what fits, 24 warps,
+    // this): planted RMAT-13 at k = 5 92..101, 83, 83; planted RMAT-15 at k = 4
+    // 45 with 24 warps, 35 so; 60,000 vertices with communities 16 and 9, and a
+    // pass takes 475 and 385 us.  A planted RMAT-12 at k = 3 has its densest set
+    // first after 64 passes in 308 of 360 runs with what fits, in 336 so (in 208
+    // of 300 when each run is certified), and its pass takes 129 and 96 us.
+    if (MODE == MODE_SEQ && a.shared_loads) {
+      const uint64_t share = std::min<uint64_t>(t.streams / (32 * (uint64_t)t.num_sms), 64);
+      per_sm = std::min(per_sm, std::max(1, (int)std::max<uint64_t>(share, 24) / nw));
+    }
     fn<<<persistent_grid(per_sm, t, 1, t.active != nullptr), nw * 32, sm, st>>>(a);
     return cudaGetLastError();
   }
